@@ -4,9 +4,12 @@
 // Compiled with -fmad=false: positions (double) and the lattice math (float) round exactly as the
 // reference's -ffp-contract=off build does, so heights carry the reference CPU path's bits.
 //
-// The kernels are ALU-bound (about 1.5k integer and float operations per cell for 8 Perlin
-// octaves, 4 bytes written). Each thread evaluates several cells of one column, so a warp covers
-// 32 consecutive columns and every store is a full 128-byte line.
+// The kernels are ALU-bound (4 bytes written per cell against some 60 float operations an octave).
+// Each thread evaluates several cells of one column, so a warp covers 32 consecutive columns and
+// every store is a full 128-byte line.
+#include <algorithm>
+#include <cmath>
+
 #include "kernels.h"
 #include "noise_math.cuh"
 
@@ -50,14 +53,27 @@ __device__ __forceinline__ float row_y(const Grid& g, const Positions& at, uint3
 // constants are computed once on the host, with the same float recurrences Fractal2 runs per
 // cell (fractal.h:219-240), so each cell performs exactly the reference's operations on them.
 constexpr int kMaxOctaves = 32;
+// Lattice points a block's tables hold in all (3 floats each): 15 KB, so shared memory does not
+// limit a block's occupancy below what its registers do.
+constexpr uint32_t kTablePoints = 1280;
+constexpr uint32_t kTableSteps = kTablePoints / 32;
 struct Octaves {
     int count;
     float amplitude;
     float total;                       // sum of the weights
+    float one;                         // 1
+    uint32_t tabled;                   // bit o: octave o reads its block's lattice table
     uint32_t seedTerm[kMaxOctaves];    // octave seed, through pcg3d's first LCG step
     float ox[kMaxOctaves], oy[kMaxOctaves];
     float frequency[kMaxOctaves], weight[kMaxOctaves];
     float tc[kMaxOctaves], ts[kMaxOctaves];
+    // A tabled octave's points: its columns and their reciprocal, how many there are, and its
+    // first point in the table, a multiple of 32: the points are hashed 32 to a warp's step, and
+    // step k of a block's `steps` belongs to octave stepOctave[k].
+    uint16_t across[kMaxOctaves], points[kMaxOctaves], first[kMaxOctaves];
+    float acrossInverse[kMaxOctaves];
+    uint32_t steps;
+    uint8_t stepOctave[kTableSteps];
 };
 
 constexpr uint32_t kLcgA = 1664525u, kLcgC = 1013904223u;
@@ -73,63 +89,266 @@ __device__ __forceinline__ uint32_t corner_from_terms(uint32_t x, uint32_t y, ui
     return x + y * z;
 }
 
-constexpr int kFbmRows = 8;  // rows per thread in the fBm kernel
+// The gradient of the lattice corner (ix, iy) of an octave.
+__device__ __forceinline__ noise::Gradient corner_gradient(uint32_t ix, uint32_t iy,
+                                                           uint32_t seedTerm) {
+    return noise::gradient_of(
+        corner_from_terms(ix * kLcgA + kLcgC, iy * kLcgA + kLcgC, seedTerm));
+}
 
-// The fBm source: octave-outer over kFbmRows cells of a column, reusing a lattice cell's four
-// corner hashes from the row above when the cell is the same (most rows, at broad octaves).
-__global__ void __launch_bounds__(kBlockX* kBlockY)
+// Adding 1.5 * 2^23 rounding down leaves floor(q) in the low bits of a float's significand, exact
+// for |q| < 2^22: the lattice cell as an integer and, subtracting it again, as a float, without
+// the conversion unit.
+constexpr float kFloorShift = 12582912.0f;
+constexpr uint32_t kFloorBits = 0x4b400000u;
+
+// Two floats (two rows of a column) in a register pair, each operation one instruction on both
+// with the same rounding as the scalar one.
+struct Pair {
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair pair_of(float a, float b) {
+    Pair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+    return p;
+}
+__device__ __forceinline__ void halves(Pair p, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ Pair both(float a) {
+    return pair_of(a, a);
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair p;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
+    return p;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair p;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return p;
+}
+// Sums and differences as a 1 + b and b (-1) + a, which round as a + b and a - b do: the
+// assembler fuses a packed product into a packed add (it leaves scalar ones alone under
+// -fmad=false), but not into a multiply-add. `one` is a kernel argument, so it stays a factor.
+struct Arithmetic {
+    Pair one, minusOne;
+    __device__ __forceinline__ explicit Arithmetic(float o) : one(both(o)), minusOne(both(-o)) {}
+    __device__ __forceinline__ Pair add(Pair a, Pair b) const { return fma2(a, one, b); }
+    __device__ __forceinline__ Pair sub(Pair a, Pair b) const { return fma2(b, minusOne, a); }
+    __device__ __forceinline__ Pair add_down(Pair a, Pair b) const {
+        Pair p;
+        asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(one.v), "l"(b.v));
+        return p;
+    }
+    __device__ __forceinline__ Pair fade(Pair t) const {  // noise::fade
+        const Pair inner =
+            add(mul2(t, sub(mul2(t, both(6.0f)), both(15.0f))), both(10.0f));
+        return mul2(mul2(mul2(t, t), t), inner);
+    }
+    __device__ __forceinline__ Pair lerp(Pair t, Pair a, Pair b) const {  // noise::lerp
+        return add(mul2(t, sub(b, a)), a);
+    }
+};
+
+// The gradients of one lattice corner of two rows' cells.
+struct GradientPair {
+    Pair x, y, s;
+};
+__device__ __forceinline__ Pair gradient_dot2(const GradientPair& g, Pair x, Pair y) {
+    return mul2(fma2(g.x, x, mul2(g.y, y)), g.s);  // noise::gradient_dot
+}
+__device__ __forceinline__ GradientPair gradient_pair(const float* table, uint32_t a, uint32_t b) {
+    return GradientPair{pair_of(table[a], table[b]),
+                        pair_of(table[kTablePoints + a], table[kTablePoints + b]),
+                        pair_of(table[2 * kTablePoints + a], table[2 * kTablePoints + b])};
+}
+
+// PerlinNoise2 (perlin.h:72-98) at fraction (fx, fy) of a cell, its corners' gradients given.
+__device__ __forceinline__ float perlin_in(const noise::Gradient (&g)[4], float fx, float fy) {
+    const float n00 = noise::gradient_dot(g[0], fx, fy);
+    const float n10 = noise::gradient_dot(g[1], fx - 1.0f, fy);
+    const float n01 = noise::gradient_dot(g[2], fx, fy - 1.0f);
+    const float n11 = noise::gradient_dot(g[3], fx - 1.0f, fy - 1.0f);
+    const float u = noise::fade(fx);
+    const float v = noise::fade(fy);
+    return 1.41421356237309505f *
+           noise::lerp(v, noise::lerp(u, n00, n10), noise::lerp(u, n01, n11));
+}
+
+// The fBm source: octave-outer over kRows cells of a column. It is bound by issuing instructions
+// and by the float pipe, so:
+//   - each octave of a block whose lattice points are few (its tile spans a few lattice cells)
+//     reads their gradients from a table the block hashes once;
+//   - the rows of such an octave run two to an instruction (Pair), 54 for two cells, and with no
+//     branch between the pairs: an octave whose rows share a cell in every lane loads its
+//     gradients once, any other loads them for every pair (cheaper than asking which changed:
+//     293 against 303 us).
+// 4097^2 cells of 8 octaves: 626 us when each thread hashed and selected its corners' gradients
+// (159 instructions a cell and octave), 338 with the tables and one row to an instruction, 293
+// now; the float operations alone take 200 us at the pipe's rate. Octaves too fine for the table
+// hash their corners per cell. Grids are not rotated (the entry points refuse others), so a
+// cell's x depends on its column alone and its y on its row alone.
+template <int kRows>
+__global__ void __launch_bounds__(kBlockX* kBlockY, 3)
     fbm_kernel(const Octaves oct, const Grid grid, const Positions at, const bool fill,
                const float elevation, const NoData nodata, float* __restrict__ heights) {
-    const uint32_t col = blockIdx.x * kBlockX + threadIdx.x;
-    const uint32_t row0 = (blockIdx.y * kBlockY + threadIdx.y) * kFbmRows;
-    if (col >= grid.width || row0 >= grid.height) {
+    static_assert(kRows % 2 == 0, "rows run in pairs");
+    __shared__ float table[3 * kTablePoints];
+    __shared__ uint32_t bases[kMaxOctaves];
+    const uint32_t tile0 = blockIdx.y * kBlockY * kRows;
+    if (oct.tabled != 0u) {
+        // The tile's corner cells bound its lattice positions: every other cell's lies between
+        // them but for rounding (below 1/8 of a lattice cell where octaves are tabled), which the
+        // margin of one point on each side covers.
+        const uint32_t c0 = blockIdx.x * kBlockX, c1 = min(c0 + kBlockX, grid.width) - 1u;
+        const uint32_t r0 = tile0, r1 = min(r0 + kBlockY * kRows, grid.height) - 1u;
+        float cx[4], cy[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t c = k & 1 ? c1 : c0, r = k & 2 ? r1 : r0;
+            cx[k] = k > 1 ? cx[k & 1] : column_x(grid, at, c, r);
+            cy[k] = k & 1 ? cy[k & 2] : row_y(grid, at, c, r);
+        }
+        for (uint32_t step = threadIdx.y; step < oct.steps; step += kBlockY) {
+            const uint32_t o = oct.stepOctave[step];
+            const uint32_t across = oct.across[o], first = oct.first[o];
+            const uint32_t p = step * 32u - first + threadIdx.x;
+            const float tc = oct.tc[o], ts = oct.ts[o], f = oct.frequency[o];
+            float qx = INFINITY, qy = INFINITY;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                qx = fminf(qx, (cx[k] * tc - cy[k] * ts) * f + oct.ox[o]);
+                qy = fminf(qy, (cx[k] * ts + cy[k] * tc) * f + oct.oy[o]);
+            }
+            const uint32_t ix0 = uint32_t(__float2int_rd(qx) - 1);
+            const uint32_t iy0 = uint32_t(__float2int_rd(qy) - 1);
+            if (p == 0u) {
+                bases[o] = first - (iy0 + kFloorBits) * across - (ix0 + kFloorBits);
+            }
+            if (p < oct.points[o]) {
+                // p / across: both below 2^11, so the half keeps the float quotient off integers.
+                const uint32_t j = uint32_t((float(p) + 0.5f) * oct.acrossInverse[o]);
+                const noise::Gradient g =
+                    corner_gradient(ix0 + p - j * across, iy0 + j, oct.seedTerm[o]);
+                float* entry = table + step * 32u + threadIdx.x;
+                entry[0] = g.x;
+                entry[kTablePoints] = g.y;
+                entry[2 * kTablePoints] = g.s;
+            }
+        }
+        __syncthreads();
+    }
+    const uint32_t row0 = tile0 + threadIdx.y * kRows;
+    if (row0 >= grid.height) {
         return;
     }
-    const int rows = min(kFbmRows, int(grid.height - row0));
-    float xs[kFbmRows], ys[kFbmRows], sum[kFbmRows];
+    // Lanes past the last column evaluate it with the others and write nothing.
+    const bool inside = blockIdx.x * kBlockX + threadIdx.x < grid.width;
+    const uint32_t col = inside ? blockIdx.x * kBlockX + threadIdx.x : grid.width - 1u;
+    const int rows = min(kRows, int(grid.height - row0));
+    constexpr int kPairs = kRows / 2;
+    const float x0 = column_x(grid, at, col, row0);
+    const Pair x = both(x0);
+    Pair ys[kPairs], sum[kPairs];
 #pragma unroll
-    for (int r = 0; r < kFbmRows; ++r) {
-        const uint32_t row = row0 + min(r, rows - 1);
-        xs[r] = column_x(grid, at, col, row);
-        ys[r] = row_y(grid, at, col, row);
-        sum[r] = 0.0f;
+    for (int k = 0; k < kPairs; ++k) {
+        const uint32_t a = row0 + min(2 * k, rows - 1), b = row0 + min(2 * k + 1, rows - 1);
+        ys[k] = pair_of(row_y(grid, at, col, a), row_y(grid, at, col, b));
+        sum[k] = both(0.0f);
     }
+    const Arithmetic on(oct.one);
     for (int o = 0; o < oct.count; ++o) {
         const float tc = oct.tc[o], ts = oct.ts[o], f = oct.frequency[o];
         const float ox = oct.ox[o], oy = oct.oy[o], w = oct.weight[o];
-        const uint32_t sz = oct.seedTerm[o];
-        int32_t cx = INT32_MIN, cy = INT32_MIN;
-        uint32_t h00 = 0, h10 = 0, h01 = 0, h11 = 0;
+        if ((oct.tabled >> o) & 1u) {
+            const uint32_t base = bases[o], across = oct.across[o];
+            Pair fx[kPairs], fy[kPairs];
+            uint32_t cells[kPairs][2];  // each row's cell's place in the table
+            bool same = true;
 #pragma unroll
-        for (int r = 0; r < kFbmRows; ++r) {
-            // Fractal2's rotation and lattice position, then PerlinNoise2 (perlin.h:72-98).
-            const float rx = xs[r] * tc - ys[r] * ts;
-            const float ry = xs[r] * ts + ys[r] * tc;
+            for (int k = 0; k < kPairs; ++k) {
+                // Fractal2's rotation and lattice position, split as split2 does.
+                const Pair y = ys[k];
+                const Pair qx = on.add(
+                    mul2(on.sub(mul2(x, both(tc)), mul2(y, both(ts))), both(f)), both(ox));
+                const Pair qy = on.add(
+                    mul2(on.add(mul2(x, both(ts)), mul2(y, both(tc))), both(f)), both(oy));
+                const Pair lx = on.add_down(qx, both(kFloorShift));
+                const Pair ly = on.add_down(qy, both(kFloorShift));
+                fx[k] = on.sub(qx, on.sub(lx, both(kFloorShift)));
+                fy[k] = on.sub(qy, on.sub(ly, both(kFloorShift)));
+                float ax, bx, ay, by;
+                halves(lx, ax, bx);
+                halves(ly, ay, by);
+                cells[k][0] = base + __float_as_uint(ay) * across + __float_as_uint(ax);
+                cells[k][1] = base + __float_as_uint(by) * across + __float_as_uint(bx);
+                same = same && cells[k][0] == cells[0][0] && cells[k][1] == cells[0][0];
+            }
+            GradientPair g00, g10, g01, g11;
+            auto load = [&](uint32_t a, uint32_t b) {
+                g00 = gradient_pair(table, a, b);
+                g10 = gradient_pair(table, a + 1u, b + 1u);
+                g01 = gradient_pair(table, a + across, b + across);
+                g11 = gradient_pair(table, a + across + 1u, b + across + 1u);
+            };
+            auto add = [&](int k) {
+                const Pair gx = on.sub(fx[k], both(1.0f)), gy = on.sub(fy[k], both(1.0f));
+                const Pair n00 = gradient_dot2(g00, fx[k], fy[k]);
+                const Pair n10 = gradient_dot2(g10, gx, fy[k]);
+                const Pair n01 = gradient_dot2(g01, fx[k], gy);
+                const Pair n11 = gradient_dot2(g11, gx, gy);
+                const Pair u = on.fade(fx[k]), v = on.fade(fy[k]);
+                const Pair n = mul2(both(1.41421356237309505f),
+                                    on.lerp(v, on.lerp(u, n00, n10), on.lerp(u, n01, n11)));
+                sum[k] = on.add(mul2(both(w), n), sum[k]);
+            };
+            load(cells[0][0], cells[0][1]);
+            if (__all_sync(0xffffffffu, same)) {
+                // Every lane's rows in one cell (broad octaves): no branch between the pairs.
+#pragma unroll
+                for (int k = 0; k < kPairs; ++k) {
+                    add(k);
+                }
+                continue;
+            }
+#pragma unroll
+            for (int k = 0; k < kPairs; ++k) {
+                if (k > 0) {
+                    load(cells[k][0], cells[k][1]);
+                }
+                add(k);
+            }
+            continue;
+        }
+        const uint32_t sz = oct.seedTerm[o];
+        noise::Gradient g[4];
+        int32_t cx = 0, cy = 0;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            float ya, yb, sa, sb;
+            halves(ys[r / 2], ya, yb);
+            halves(sum[r / 2], sa, sb);
+            const float y = r & 1 ? yb : ya;
+            const float rx = x0 * tc - y * ts;
+            const float ry = x0 * ts + y * tc;
             const noise::Cell2 c = noise::split2(rx * f + ox, ry * f + oy);
-            if (c.ix != cx || c.iy != cy) {
+            if (r == 0 || c.ix != cx || c.iy != cy) {
                 cx = c.ix;
                 cy = c.iy;
-                const uint32_t ax0 = uint32_t(c.ix) * kLcgA + kLcgC, ax1 = ax0 + kLcgA;
-                const uint32_t ay0 = uint32_t(c.iy) * kLcgA + kLcgC, ay1 = ay0 + kLcgA;
-                h00 = corner_from_terms(ax0, ay0, sz);
-                h10 = corner_from_terms(ax1, ay0, sz);
-                h01 = corner_from_terms(ax0, ay1, sz);
-                h11 = corner_from_terms(ax1, ay1, sz);
+                const uint32_t x0 = uint32_t(c.ix), y0 = uint32_t(c.iy);
+                g[0] = corner_gradient(x0, y0, sz);
+                g[1] = corner_gradient(x0 + 1u, y0, sz);
+                g[2] = corner_gradient(x0, y0 + 1u, sz);
+                g[3] = corner_gradient(x0 + 1u, y0 + 1u, sz);
             }
-            const float n00 = noise::gradient2(h00, c.fx, c.fy);
-            const float n10 = noise::gradient2(h10, c.fx - 1.0f, c.fy);
-            const float n01 = noise::gradient2(h01, c.fx, c.fy - 1.0f);
-            const float n11 = noise::gradient2(h11, c.fx - 1.0f, c.fy - 1.0f);
-            const float u = noise::fade(c.fx);
-            const float v = noise::fade(c.fy);
-            const float n = 1.41421356237309505f *
-                            noise::lerp(v, noise::lerp(u, n00, n10), noise::lerp(u, n01, n11));
-            sum[r] += w * n;
+            const float add = w * perlin_in(g, c.fx, c.fy);
+            sum[r / 2] = r & 1 ? pair_of(sa, sb + add) : pair_of(sa + add, sb);
         }
     }
 #pragma unroll
-    for (int r = 0; r < kFbmRows; ++r) {
-        if (r >= rows) {
+    for (int r = 0; r < kRows; ++r) {
+        if (r >= rows || !inside) {
             break;
         }
         const size_t i = size_t(row0 + r) * grid.width + col;
@@ -141,8 +360,65 @@ __global__ void __launch_bounds__(kBlockX* kBlockY)
             }
         }
         // EvaluateFractals of one enabled fractal: amplitude * (1 * sum / total).
-        heights[i] = base + oct.amplitude * (1.0f * sum[r] / oct.total);
+        float sa, sb;
+        halves(sum[r / 2], sa, sb);
+        heights[i] = base + oct.amplitude * (1.0f * (r & 1 ? sb : sa) / oct.total);
     }
+}
+
+// Which octaves a block of kBlockX columns by `tileRows` rows reads from its table, and where:
+// those whose lattice box over the tile fits what is left of the table, coarsest first, with
+// every lattice position of the grid below 2^18 (so that the float positions are good to 1/8 and
+// kFloorShift is exact). Positions from arrays are not bounded by a tile's corners: none.
+void place_tables(Octaves& oct, const Grid& g, const Positions& at, uint32_t tileRows) {
+    oct.tabled = 0u;
+    oct.steps = 0u;
+    if (at.xs != nullptr || at.ys != nullptr) {
+        return;
+    }
+    double reach = 0.0;  // the largest |x| + |y| of a cell center
+    for (int k = 0; k < 4; ++k) {
+        const double c = k & 1 ? double(g.width) : 0.0, r = k & 2 ? double(g.height) : 0.0;
+        const double x = g.originX + c * g.pixelWidth + r * g.rowRotation - at.originX;
+        const double y = g.originY + c * g.colRotation + r * g.pixelHeight - at.originY;
+        reach = std::max(reach, std::fabs(x) + std::fabs(y));
+    }
+    const double spanC = double(kBlockX - 1), spanR = double(tileRows - 1);
+    const double wide = spanC * std::fabs(g.pixelWidth) + spanR * std::fabs(g.rowRotation);
+    const double high = spanC * std::fabs(g.colRotation) + spanR * std::fabs(g.pixelHeight);
+    for (int o = 0; o < oct.count; ++o) {
+        const double f = std::fabs(double(oct.frequency[o]));
+        const double tc = std::fabs(double(oct.tc[o])), ts = std::fabs(double(oct.ts[o]));
+        if (!(reach * f < 262144.0)) {
+            continue;
+        }
+        // The box's cells, their far corners, the margin on each side and one for rounding.
+        const double across = std::floor((wide * tc + high * ts) * f) + 5.0;
+        const double down = std::floor((wide * ts + high * tc) * f) + 5.0;
+        if (!(across * down <= double((kTableSteps - oct.steps) * 32u))) {
+            continue;
+        }
+        oct.tabled |= 1u << o;
+        oct.first[o] = uint16_t(oct.steps * 32u);
+        oct.across[o] = uint16_t(across);
+        oct.acrossInverse[o] = 1.0f / float(across);
+        oct.points[o] = uint16_t(across * down);
+        for (uint32_t p = 0; p < oct.points[o]; p += 32u) {
+            oct.stepOctave[oct.steps++] = uint8_t(o);
+        }
+    }
+}
+
+template <int kRows>
+void launch_fbm(Octaves& oct, const Grid& grid, const Positions& at, bool fill, float elevation,
+                NoData nodata, float* heights, cudaStream_t stream) {
+    const uint32_t rowsPerBlock = kBlockY * kRows;
+    place_tables(oct, grid, at, rowsPerBlock);
+    const dim3 block(kBlockX, kBlockY);
+    const dim3 blocks((grid.width + kBlockX - 1) / kBlockX,
+                      (grid.height + rowsPerBlock - 1) / rowsPerBlock);
+    fbm_kernel<kRows><<<blocks, block, 0, stream>>>(oct, grid, at, fill, elevation, nodata,
+                                                    heights);
 }
 
 // Any stack of fractals (bases, types, blends, warps), cell by cell.
@@ -299,10 +575,18 @@ cudaError_t launch_noise(const FractalStack& stack, const Grid& grid, const Posi
             tc = nc;
         }
         oct.total = total;
-        const uint32_t rowsPerBlock = kBlockY * kFbmRows;
-        const dim3 blocks((grid.width + kBlockX - 1) / kBlockX,
-                          (grid.height + rowsPerBlock - 1) / rowsPerBlock);
-        fbm_kernel<<<blocks, block, 0, stream>>>(oct, grid, at, fill, elevation, nodata, heights);
+        oct.one = 1.0f;
+        // Rows a thread takes: 8 amortize a block's tables best (2049^2 cells: 81 us against 106
+        // with 2), as long as that leaves the SMs several blocks each; a small grid's octaves
+        // run in parallel over its cells instead of in series over a few blocks (257^2: the
+        // kernel took 17 us with 8 rows a thread; with 2 the whole call takes 12).
+        const size_t columns = (grid.width + kBlockX - 1) / kBlockX;
+        const size_t lines = (grid.height + kBlockY - 1) / kBlockY;
+        if (columns * lines >= 8 * 1184) {
+            launch_fbm<8>(oct, grid, at, fill, elevation, nodata, heights, stream);
+        } else {
+            launch_fbm<2>(oct, grid, at, fill, elevation, nodata, heights, stream);
+        }
         return cudaGetLastError();
     }
     const uint32_t rowsPerBlock = kBlockY * kRowsPerThread;

@@ -83,6 +83,29 @@ __device__ __forceinline__ float gradient2(uint32_t hash, float x, float y) {
     return h < 4u ? ((h & 1u) != 0u ? -axis : axis) : diagonal;
 }
 
+// The gradient a corner hash picks, as coefficients: gradient2(hash, x, y) is
+// (x gx + y gy) s, with gx, gy in {0, 2, -2} and s 1/2 or 1 / (2 sqrt 2). The coefficients' top
+// bytes (0x40 for 2, 0xc0 for -2, 0 for 0) come from eight-entry byte tables held in the operands
+// of a byte permute, indexed by the hash's three low bits.
+struct Gradient {
+    float x, y, s;
+};
+__device__ __forceinline__ Gradient gradient_of(uint32_t hash) {
+    const uint32_t pick = (hash << 12u) & 0x7000u;
+    Gradient g;
+    g.x = __uint_as_float(__byte_perm(0x0000c040u, 0xc040c040u, pick | 0x222u));
+    g.y = __uint_as_float(__byte_perm(0xc0400000u, 0xc0c04040u, pick));
+    g.s = (hash & 4u) != 0u ? 0.5f * 0.707106781186547524f : 0.5f;
+    return g;
+}
+
+// gradient2 from the coefficients, three operations instead of gradient2's selects: y gy is
+// exact, so the fused sum rounds x gx + y gy once, as the selects' sum does; a zero may differ in
+// sign, which no interpolation or octave sum keeps (sums start at +0).
+__device__ __forceinline__ float gradient_dot(const Gradient& g, float x, float y) {
+    return fmaf(g.x, x, g.y * y) * g.s;
+}
+
 // Hash of a 2D lattice corner keyed (x, y, seed) (perlin.h:31, lattice.h:94).
 __device__ __forceinline__ uint32_t corner2(uint32_t ix, uint32_t iy, uint32_t seed) {
     return pcg3d(U3{ix, iy, seed}).x;
