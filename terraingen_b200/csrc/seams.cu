@@ -14,7 +14,7 @@
 //   3b. Height / Slope: gap posts within the reach (3 decay lengths, away from the lattice's 3
 //      border posts) are solved for (-Laplacian + 1/L^2) d = 0, or its square, with the band's
 //      values fixed: conjugate gradients in FP64 preconditioned by a symmetric multigrid V-cycle
-//      (damped Jacobi smoothing in FP32, the coarsest level's residual and sweeps in FP64) over
+//      (Chebyshev smoothing in FP32, the coarsest level's residual and sweeps in FP64) over
 //      the unknowns compacted on each level. The reference solves the same system per connected
 //      region with Gauss-Seidel smoothing; the converged field is the same.
 // The field is read between posts by Catmull-Rom interpolation (SeamField::At) when a grid's
@@ -565,16 +565,41 @@ __global__ void active_tiles_kernel(const uint32_t* __restrict__ counts, uint32_
 // count of unknowns before its word (an exclusive scan of the words' counts) plus those before
 // it in the word.
 
-// A coarser level's posts: the parents (col / 2, row / 2) of the finer level's unknowns.
-__global__ void coarsen_kernel(const uint32_t* __restrict__ finePos, uint32_t n, uint32_t fineW,
-                               uint32_t coarsePitch, uint32_t* __restrict__ coarseMask) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) {
+// The finer unknowns' bits of columns 64 q .. 64 q + 63 that are the left one of a pair (columns
+// 2 c, 2 c + 1) both unknown, packed 32 pairs to a word.
+__device__ __forceinline__ uint32_t whole_pairs(uint32_t low, uint32_t high) {
+    auto squeeze = [](uint32_t v) {  // the even bits, packed into the low half
+        v &= v >> 1;
+        v &= 0x55555555u;
+        v = (v | (v >> 1)) & 0x33333333u;
+        v = (v | (v >> 2)) & 0x0f0f0f0fu;
+        v = (v | (v >> 4)) & 0x00ff00ffu;
+        return (v | (v >> 8)) & 0x0000ffffu;
+    };
+    return squeeze(low) | (squeeze(high) << 16);
+}
+
+// A coarser level's posts: (C, R) where all four finer posts (2 C, 2 C + 1) x (2 R, 2 R + 1) are
+// unknowns. Coarse posts that overhang the finer unknowns' border (parents of any of them, as
+// BuildHierarchy takes) move the fixed border outward by up to a post a level, and the correction
+// they give near it is wrong: over a ring 64 posts wide the conjugate gradients took 18
+// iterations (Height) and over 200 (Slope) with them, 14 and 46 without, with the same sweeps.
+__global__ void coarsen_kernel(const uint32_t* __restrict__ fine, uint32_t finePitch,
+                               uint32_t fineH, uint32_t coarsePitch, uint32_t coarseH,
+                               uint32_t* __restrict__ coarseMask) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= coarsePitch * coarseH) {
         return;
     }
-    const uint32_t p = finePos[k];
-    const uint32_t col = (p % fineW) / 2, row = p / fineW / 2;
-    atomicOr(&coarseMask[size_t(row) * coarsePitch + (col >> 5)], 1u << (col & 31u));
+    const uint32_t row = 2u * (j / coarsePitch), word = 2u * (j % coarsePitch);
+    uint32_t both = 0;
+    if (row + 1u < fineH) {
+        const uint32_t* a = fine + size_t(row) * finePitch + word;
+        const uint32_t* b = a + finePitch;
+        const bool second = word + 1u < finePitch;
+        both = whole_pairs(a[0] & b[0], second ? a[1] & b[1] : 0u);
+    }
+    coarseMask[j] = both;
 }
 
 __global__ void word_counts_kernel(const uint32_t* __restrict__ mask, size_t words,
@@ -779,22 +804,40 @@ __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Damped Jacobi: xn = x + omega (b - A x) / diagonal; from x = 0 when `x` is null.
+// Chebyshev iteration for A x = b over the operator's eigenvalues in [low, high] (the first-kind
+// polynomial, in its three-term form): each step's weights of the last change and of the residual.
+struct ChebyshevStep {
+    double alpha, beta, rho;
+};
+struct Chebyshev {
+    double center, half;
+    __host__ __device__ ChebyshevStep first() const {
+        return ChebyshevStep{0.0, 1.0 / center, half / center};
+    }
+    __host__ __device__ ChebyshevStep next(const ChebyshevStep& s) const {
+        const double rho = 1.0 / (2.0 * center / half - s.rho);
+        return ChebyshevStep{rho * s.rho, 2.0 * rho / half, rho};
+    }
+};
+
+// One Chebyshev step: xn = x + alpha (x - before) + beta (b - A x), `before` the iterate before x
+// (null: 0) and `x` null for the step from 0. xn may be `before`: each thread reads only its own
+// value of it.
 template <int kOrder, typename T>
-__global__ void jacobi_kernel(const LevelView L, const T* __restrict__ b, const T* __restrict__ x,
-                              T* __restrict__ xn, double omega, const CgState* cg) {
+__global__ void chebyshev_kernel(const LevelView L, const T* __restrict__ b, const T* x,
+                                 const T* before, T* xn, T alpha, T beta, const CgState* cg) {
     pdl_begin();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= L.n || stopped(cg)) {
         return;
     }
-    const T scale = T(omega / L.diagonal);
     if (x == nullptr) {
-        xn[k] = scale * b[k];
+        xn[k] = beta * b[k];
         return;
     }
     const T r = b[k] - apply_at<kOrder, T, T>(L, x, k);
-    xn[k] = x[k] + scale * r;
+    const T last = before == nullptr ? T(0) : before[k];
+    xn[k] = x[k] + alpha * (x[k] - last) + beta * r;
 }
 
 template <int kOrder, typename T>
@@ -1013,15 +1056,16 @@ __global__ void cg_direction_kernel(double* __restrict__ p, const T* __restrict_
     }
 }
 
-// The coarsest level's sweeps in one block, its iterates in shared memory: the same damped
-// Jacobi steps as jacobi_kernel, a block barrier between sweeps.
+// The coarsest level's sweeps in one block, its iterates in shared memory: the same steps as
+// chebyshev_kernel, a block barrier between them.
 constexpr uint32_t kCoarsestBlockPosts = 4096;
 
 template <int kOrder>
 __global__ void __launch_bounds__(1024) coarsest_kernel(const LevelView L,
                                                         const double* __restrict__ b,
-                                                        double* __restrict__ x, double omega,
-                                                        int sweeps, const CgState* cg) {
+                                                        double* __restrict__ x,
+                                                        const Chebyshev steps, int sweeps,
+                                                        const CgState* cg) {
     pdl_begin();
     if (stopped(cg)) {
         return;
@@ -1029,20 +1073,22 @@ __global__ void __launch_bounds__(1024) coarsest_kernel(const LevelView L,
     extern __shared__ double iterates[];
     double* cur = iterates;
     double* next = iterates + L.n;
-    const double scale = omega / L.diagonal;
+    ChebyshevStep step = steps.first();
     for (int i = 0; i < sweeps; ++i) {
         for (uint32_t k = threadIdx.x; k < L.n; k += blockDim.x) {
             if (i == 0) {
-                next[k] = scale * b[k];
+                next[k] = step.beta * b[k];
             } else {
                 const double r = b[k] - apply_at<kOrder, double, double>(L, cur, k);
-                next[k] = cur[k] + scale * r;
+                const double last = i == 1 ? 0.0 : next[k];
+                next[k] = cur[k] + step.alpha * (cur[k] - last) + step.beta * r;
             }
         }
         __syncthreads();
         double* t = cur;
         cur = next;
         next = t;
+        step = steps.next(step);
     }
     for (uint32_t k = threadIdx.x; k < L.n; k += blockDim.x) {
         x[k] = cur[k];
@@ -1358,27 +1404,55 @@ struct Solver {
     int levels;
     int order;
     cudaStream_t s;
-    double omega;
     int sweeps, coarsest;
     const CgState* cg;     // the device state iterations stop on (null: always run)
     cudaStream_t capture;  // a stream of the library's own, the iterations are captured on
 };
 
+// The eigenvalues a level's sweeps act on. The operator's lie within (1/L^2)^order and
+// (center + 2 cx + 2 cy)^order (a principal submatrix of the lattice's). A smoother of n sweeps
+// takes the part that the coarser level does not represent and what n sweeps can reach below it,
+// down to 1/3n (Height) or 1/8n (Slope) of the largest: over a ring 64 posts wide, with 2 sweeps,
+// 12 iterations (14 with damped Jacobi sweeps) and 25 (46), within one of the best fraction. The
+// coarsest level takes all of them that n sweeps can reduce, the largest over 3/4 n^2 and up.
+Chebyshev smoothing(const LevelView& L, int order, int sweeps, bool coarsest) {
+    const double widest = L.center + 2.0 * L.cx + 2.0 * L.cy;
+    const double least = L.center - 2.0 * L.cx - 2.0 * L.cy;
+    const double high = order == 1 ? widest : widest * widest;
+    double low;
+    if (coarsest) {
+        low = std::max(order == 1 ? least : least * least,
+                       high / std::max(0.75 * sweeps * sweeps, 3.0));
+    } else {
+        low = high / ((order == 1 ? 3.0 : 8.0) * sweeps);
+    }
+    return Chebyshev{0.5 * (high + low), 0.5 * (high - low)};
+}
+
 double* cg_dots(CgState* cg) {
     return reinterpret_cast<double*>(reinterpret_cast<char*>(cg) + offsetof(CgState, dots));
 }
 
-template <int kOrder>
-cudaError_t jacobi(const Solver& sv, const LevelView& L, const void* b, const void* x, void* xn,
-                   bool coarsest) {
-    if (coarsest) {
-        TG_PDL_E(jacobi_kernel<kOrder, double>, blocks_for(L.n), 256, 0, sv.s,
-            L, static_cast<const double*>(b), static_cast<const double*>(x),
-            static_cast<double*>(xn), sv.omega, sv.cg);
-    } else {
-        TG_PDL_E(jacobi_kernel<kOrder, float>, blocks_for(L.n), 256, 0, sv.s,
-            L, static_cast<const float*>(b), static_cast<const float*>(x),
-            static_cast<float*>(xn), sv.omega, sv.cg);
+// A level's sweeps: from 0 or from the iterate in x, `done` of them (0 or 1) behind; the last
+// lands in x or, for sweeps from x with an odd count, in t.
+template <int kOrder, typename T>
+cudaError_t sweep(const Solver& sv, Level& L, int sweeps, bool fromZero, int done, bool coarsest) {
+    const Chebyshev c = smoothing(L.view, kOrder, sweeps, coarsest);
+    T* const x = static_cast<T*>(L.x.ptr);
+    T* const t = static_cast<T*>(L.t.ptr);
+    T* cur = fromZero ? (sweeps % 2 == 0 ? x : t) : x;  // where the iterate before sweep 0 stands
+    ChebyshevStep step = c.first();
+    for (int i = 0; i < sweeps; ++i) {
+        T* const next = cur == x ? t : x;
+        if (i >= done) {
+            const T* from = fromZero && i == 0 ? nullptr : cur;
+            const T* before = i == 0 || (fromZero && i == 1) ? nullptr : next;
+            TG_PDL_E(chebyshev_kernel<kOrder, T>, blocks_for(L.view.n), 256, 0, sv.s, L.view,
+                     static_cast<const T*>(L.b.ptr), from, before, next, T(step.alpha),
+                     T(step.beta), sv.cg);
+        }
+        cur = next;
+        step = c.next(step);
     }
     return cudaGetLastError();
 }
@@ -1418,19 +1492,15 @@ int vcycle(Solver& sv, int d, int smoothed = 0) {
         const uint32_t threads = std::min<uint32_t>(1024, (L.view.n + 31) / 32 * 32);
         TG_PDL(coarsest_kernel<kOrder>, 1, threads, size_t(L.view.n) * 16, sv.s,
             L.view, static_cast<const double*>(L.b.ptr), static_cast<double*>(L.x.ptr),
-            sv.omega, sweeps, sv.cg);
+            smoothing(L.view, kOrder, sweeps, true), sweeps, sv.cg);
         TG_CUDA(cudaGetLastError(), "coarsest launch");
         return TG_OK;
     }
-    void* cur = smoothed > 0 ? first_sweep_target(L, sweeps) : nullptr;
-    for (int i = smoothed; i < sweeps; ++i) {
-        void* next = (sweeps - i) % 2 == 1 ? L.x.ptr : L.t.ptr;
-        TG_CUDA(jacobi<kOrder>(sv, L.view, L.b.ptr, cur, next, last), "jacobi");
-        cur = next;
-    }
     if (last) {
+        TG_CUDA((sweep<kOrder, double>(sv, L, sweeps, true, smoothed, true)), "sweeps");
         return TG_OK;
     }
+    TG_CUDA((sweep<kOrder, float>(sv, L, sweeps, true, smoothed, false)), "sweeps");
     Level& C = sv.wk->levels[d + 1];
     const bool coarseLast = d + 2 == sv.levels;
     // residual into t, restricted into the coarse b
@@ -1460,11 +1530,7 @@ int vcycle(Solver& sv, int d, int smoothed = 0) {
             sv.cg);
     }
     TG_CUDA(cudaGetLastError(), "prolong launch");
-    for (int i = 0; i < sv.sweeps; ++i) {
-        TG_CUDA(jacobi<kOrder>(sv, L.view, L.b.ptr, i % 2 == 0 ? L.x.ptr : L.t.ptr,
-                               i % 2 == 0 ? L.t.ptr : L.x.ptr, false),
-                "jacobi");
-    }
+    TG_CUDA((sweep<kOrder, float>(sv, L, sv.sweeps, false, 0, false)), "sweeps");
     if (sv.sweeps % 2 == 1) {
         TG_CUDA(copy_level(sv, L.t.ptr, L.x.ptr, L.view.n, false), "copy");
     }
@@ -1542,7 +1608,7 @@ int iteration(Solver& sv, CgState* cg) {
         TG_CUDA(cudaGetLastError(), "iteration launch");
         return TG_OK;
     }
-    const float scale = float(sv.omega / L0.view.diagonal);
+    const float scale = float(smoothing(L0.view, kOrder, sv.sweeps, false).first().beta);
     TG_PDL(cg_update_kernel, blocks_for(n), 256, 0, sv.s,
         x, r, p, ap, n, static_cast<float*>(L0.b.ptr),
         static_cast<float*>(first_sweep_target(L0, sv.sweeps)), scale, cg);
@@ -1847,9 +1913,8 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
             ldx *= 2.0;
             ldy *= 2.0;
             TG_CUDA(L.mask.reserve(size_t(lp) * lh * 4), "allocation");
-            TG_CUDA(cudaMemsetAsync(L.mask.ptr, 0, size_t(lp) * lh * 4, s), "memset");
-            coarsen_kernel<<<blocks_for(F.view.n), 256, 0, s>>>(
-                F.view.position, F.view.n, F.view.w, lp, static_cast<uint32_t*>(L.mask.ptr));
+            coarsen_kernel<<<blocks_for(size_t(lp) * lh), 256, 0, s>>>(
+                F.view.mask, F.view.pitch, F.view.h, lp, lh, static_cast<uint32_t*>(L.mask.ptr));
             TG_CUDA(cudaGetLastError(), "coarsen launch");
         }
         if (int st = compact(wk, L, lw, lh, lp, s)) {
@@ -1864,6 +1929,9 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
                                            2.0 * L.view.cy * L.view.cy;
         if (levels == 0 && L.view.n == 0) {
             return finish(TG_OK);
+        }
+        if (L.view.n == 0) {
+            break;  // no whole coarse post: the level before is the coarsest
         }
         if (L.view.n <= 32u || lw < 4 || lh < 4) {  // the coarsest, as kCoarsestPosts
             ++levels;
@@ -1934,8 +2002,7 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
                                      int(kCoarsestBlockPosts * 16)),
                 "shared memory attribute");
     }
-    Solver sv{&wk, levels, order, s, order == 1 ? 0.8 : 0.5, int(o.sweeps),
-              int(o.coarsest_sweeps), nullptr, d->stream};
+    Solver sv{&wk, levels, order, s, int(o.sweeps), int(o.coarsest_sweeps), nullptr, d->stream};
     int iterations = 0;
     const double tolerance = o.tolerance > 0.0 ? o.tolerance : 1e-10;
     const int st = order == 1 ? solve<1>(sv, tolerance, 200, &iterations)
