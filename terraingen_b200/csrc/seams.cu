@@ -53,7 +53,9 @@ constexpr size_t kScratchBytes = size_t(1) << 30;  // the distance warps' stored
 // 32 j .. 32 j + 31 (bit = column % 32), `pitch` = ceil(w / 32) words a row, the bits past the
 // last column 0.
 
-constexpr int kBandRows = 16;  // rows of a band warp's span
+// Rows of a band warp's span: few, so that the lattices of small patches still fill the SMs (a
+// 2726^2 lattice: 85 us at 16 rows, with 520 warps bound by their own loads in turn; 53 at 4).
+constexpr int kBandRows = 4;
 
 __device__ __forceinline__ uint32_t row_tail_mask(uint32_t j, uint32_t pitch, uint32_t w) {
     return j + 1 == pitch && (w & 31u) != 0 ? (1u << (w & 31u)) - 1u : 0xffffffffu;
@@ -202,6 +204,11 @@ __global__ void band_bits_kernel(const BandBits p) {
 // read back. Only tiles that hold a post without data and see a post with data within their halo
 // are computed.
 //
+// The kernel is bound by the latency of its steps, some 2600 in series a tile, with two or three
+// warps an SM. Its steps therefore select instead of branching and read their data bits from
+// shared memory: a 2726^2 lattice with a 64-post halo (328 tiles) 557 -> 285 us, of which the
+// staged bits alone gave 64.
+//
 // One warp runs a tile's window. The forward pass reads the left, upper-left, upper and
 // upper-right posts: the warp takes the window's rows 32 at a time (lane = row), lane l at column
 // t - 2 l on step t, so the row above has just passed the three columns a post reads, and they
@@ -222,6 +229,7 @@ struct DistanceWarps {
     int ts;                // tile side, a multiple of 32
     int mx, my;            // halo columns and rows
     int rowFloats;         // floats of a warp's row in shared memory (or in `rows`)
+    int stageWords;        // words of a row's data bits in shared memory
     uint32_t tilesX;
     const uint32_t* list;
     const uint32_t* count;
@@ -252,6 +260,12 @@ __global__ void __launch_bounds__(32 * kDistanceWarps)
     float* rowF = kSharedRows ? smem + size_t(warp) * p.rowFloats * (kCarried ? 2 : 1)
                               : p.rows + size_t(slot) * p.rowFloats * (kCarried ? 2 : 1);
     float* rowC = rowF + p.rowFloats;
+    // With kSharedRows, a band's data bits too, word by word, a lane a row: a step's word comes
+    // from here, so that the lanes' reads, one or two of them every other step, do not each make
+    // the warp wait for L2.
+    uint32_t* const staged = reinterpret_cast<uint32_t*>(
+                                 smem + size_t(kDistanceWarps) * p.rowFloats * (kCarried ? 2 : 1)) +
+                             size_t(warp) * p.stageWords * 32 + lane;
     float* store = p.scratch + size_t(slot) * p.scratchFloats;
     const float inf = INFINITY;
     const uint32_t total = *p.count;
@@ -260,272 +274,235 @@ __global__ void __launch_bounds__(32 * kDistanceWarps)
         const int r0 = int(tile / p.tilesX) * p.ts, c0 = int(tile % p.tilesX) * p.ts;
         const int rw0 = max(0, r0 - p.my), rw1 = min(int(p.h), r0 + p.ts + p.my);
         const int cw0 = max(0, c0 - p.mx), cw1 = min(int(p.w), c0 + p.ts + p.mx);
-        const int ww = cw1 - cw0, steps = ww + 62;
+        const int ww = cw1 - cw0, steps = (ww + 62 + kGroup - 1) / kGroup * kGroup;
+        const int firstWord = cw0 >> 5, words = ((cw1 - 1) >> 5) - firstWord + 1;
         const int bandsAbove = (r0 - rw0 + 31) / 32, bandsBelow = (rw1 - r0 + 31) / 32;
         const int tr1 = min(int(p.h), r0 + p.ts), tc1 = min(int(p.w), c0 + p.ts);
         float* storeC = store + size_t(bandsBelow) * steps * 32;
-        for (int c = lane; c < ww; c += 32) {
-            rowF[c] = inf;
-            if (kCarried) rowC[c] = 0.0f;
-        }
-        __syncwarp();
+        // Column c of the window, of this lane's row: whether it has data (rows' bits staged in
+        // shared memory by the band, or read from the mask).
+        size_t rowBits = 0;
+        bool active = false;
+        auto stage = [&]() {
+            if (kSharedRows) {
+                for (int i = 0; i < words; ++i) {
+                    staged[i * 32] = active ? p.bits[rowBits + uint32_t(firstWord + i)] : 0u;
+                }
+            }
+        };
+        auto has_data = [&](int x) -> bool {
+            const int i = min(max((x >> 5) - firstWord, 0), words - 1);
+            const uint32_t word = kSharedRows ? staged[i * 32]
+                                  : active    ? p.bits[rowBits + uint32_t(firstWord + i)]
+                                              : 0u;
+            return (word >> (x & 31)) & 1u;
+        };
+        // Relaxes (d, car) through a neighbor (of distance `from` and carried value `carFrom`) a
+        // step away, if that is nearer.
+        auto relax = [&](float& d, float& car, float from, float carFrom, float step) {
+            const float through = from + step;
+            if (kCarried) {
+                car = through < d ? carFrom : car;
+            }
+            d = fminf(through, d);
+        };
+        auto clear_rows = [&]() {
+            for (int c = lane; c < ww; c += 32) {
+                rowF[c] = inf;
+                if (kCarried) rowC[c] = 0.0f;
+            }
+            __syncwarp();
+        };
+        clear_rows();
         // Forward, bands top down.
         for (int band = -bandsAbove; band < bandsBelow; ++band) {
             const int row = r0 + 32 * band + lane;
-            const bool active = row >= rw0 && row < rw1;
-            const size_t rowBits = size_t(active ? row : rw0) * p.pitch;
+            active = row >= rw0 && row < rw1;
+            rowBits = size_t(active ? row : rw0) * p.pitch;
+            const size_t rowField = size_t(active ? row : rw0) * p.w;
             float h1 = inf, h2 = inf, h3 = inf;
             float g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
-            uint32_t word = 0, next = 0;
-            if (active) {
-                word = p.bits[rowBits + uint32_t(cw0 >> 5)];
-                next = (cw0 >> 5) + 1 < int(p.pitch) ? p.bits[rowBits + uint32_t(cw0 >> 5) + 1]
-                                                     : 0u;
-            }
-            float* out = store + size_t(max(band, 0)) * steps * 32;
-            float* outC = storeC + size_t(max(band, 0)) * steps * 32;
+            stage();
+            float* out = store + size_t(max(band, 0)) * steps * 32 + lane;
+            float* outC = storeC + size_t(max(band, 0)) * steps * 32 + lane;
             for (int t0 = 0; t0 < steps; t0 += kGroup) {
-            // Lane 0's row above over the group's columns t0 - 1 .. t0 + kGroup, read at once
-            // (lane 31 of this band writes only columns left of them meanwhile).
-            float above[kGroup + 2], aboveC[kGroup + 2];
-            if (lane == 0) {
+                // Lane 0's row above over the group's columns t0 - 1 .. t0 + kGroup, and the
+                // lane's own columns' data bits and values, read at once (lane 31 of this band
+                // writes only columns left of lane 0's meanwhile).
+                float above[kGroup + 2], aboveC[kGroup + 2], value[kGroup];
+                bool has[kGroup];
 #pragma unroll
                 for (int i = 0; i < kGroup + 2; ++i) {
                     const int col = t0 - 1 + i;
-                    const bool in = col >= 0 && col < ww;
+                    const bool in = lane == 0 && col >= 0 && col < ww;
                     above[i] = in ? rowF[col] : inf;
                     if (kCarried) aboveC[i] = in ? rowC[col] : 0.0f;
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < kGroup; ++u) {
-                const int t = t0 + u;
-                if (t >= steps) {
-                    break;
-                }
-                const int c = t - 2 * lane;
-                float uR = __shfl_up_sync(0xffffffffu, h1, 1);
-                float uU = __shfl_up_sync(0xffffffffu, h2, 1);
-                float uL = __shfl_up_sync(0xffffffffu, h3, 1);
-                float vR = 0.0f, vU = 0.0f, vL = 0.0f;
-                if (kCarried) {
-                    vR = __shfl_up_sync(0xffffffffu, g1, 1);
-                    vU = __shfl_up_sync(0xffffffffu, g2, 1);
-                    vL = __shfl_up_sync(0xffffffffu, g3, 1);
-                }
-                if (lane == 0) {
-                    uL = above[u];
-                    uU = above[u + 1];
-                    uR = above[u + 2];
+                for (int u = 0; u < kGroup; ++u) {
+                    const int c = t0 + u - 2 * lane;
+                    has[u] = has_data(cw0 + c) && active && c >= 0 && c < ww;
                     if (kCarried) {
-                        vL = aboveC[u];
-                        vU = aboveC[u + 1];
-                        vR = aboveC[u + 2];
+                        value[u] = has[u] ? p.field[rowField + uint32_t(cw0 + c)] : 0.0f;
                     }
                 }
-                float d = inf, car = 0.0f;
-                if (active && c >= 0 && c < ww) {
-                    const int x = cw0 + c;
-                    if ((x & 31) == 0 && c > 0) {
-                        word = next;
-                        next = (x >> 5) + 1 < int(p.pitch) ? p.bits[rowBits + uint32_t(x >> 5) + 1]
-                                                           : 0u;
+#pragma unroll
+                for (int u = 0; u < kGroup; ++u) {
+                    const int t = t0 + u;
+                    const int c = t - 2 * lane;
+                    float uR = __shfl_up_sync(0xffffffffu, h1, 1);
+                    float uU = __shfl_up_sync(0xffffffffu, h2, 1);
+                    float uL = __shfl_up_sync(0xffffffffu, h3, 1);
+                    float vR = 0.0f, vU = 0.0f, vL = 0.0f;
+                    if (kCarried) {
+                        vR = __shfl_up_sync(0xffffffffu, g1, 1);
+                        vU = __shfl_up_sync(0xffffffffu, g2, 1);
+                        vL = __shfl_up_sync(0xffffffffu, g3, 1);
                     }
-                    if ((word >> (x & 31)) & 1u) {
-                        d = 0.0f;
-                        if (kCarried) car = p.field[size_t(row) * p.w + uint32_t(x)];
-                    } else {
-                        float s = h1 + p.dx;
-                        if (s < d) {
-                            d = s;
-                            car = g1;
-                        }
-                        s = uU + p.dy;
-                        if (s < d) {
-                            d = s;
-                            car = vU;
-                        }
-                        s = uL + p.diagonal;
-                        if (s < d) {
-                            d = s;
-                            car = vL;
-                        }
-                        s = uR + p.diagonal;
-                        if (s < d) {
-                            d = s;
-                            car = vR;
-                        }
+                    uL = lane == 0 ? above[u] : uL;
+                    uU = lane == 0 ? above[u + 1] : uU;
+                    uR = lane == 0 ? above[u + 2] : uR;
+                    if (kCarried) {
+                        vL = lane == 0 ? aboveC[u] : vL;
+                        vU = lane == 0 ? aboveC[u + 1] : vU;
+                        vR = lane == 0 ? aboveC[u + 2] : vR;
                     }
-                    if (lane == 31) {
+                    const bool in = active && c >= 0 && c < ww;
+                    float d = inf, car = 0.0f;
+                    relax(d, car, h1, g1, p.dx);
+                    relax(d, car, uU, vU, p.dy);
+                    relax(d, car, uL, vL, p.diagonal);
+                    relax(d, car, uR, vR, p.diagonal);
+                    d = !in ? inf : has[u] ? 0.0f : d;
+                    if (kCarried) car = !in ? 0.0f : has[u] ? value[u] : car;
+                    if (in && lane == 31) {
                         rowF[c] = d;
                         if (kCarried) rowC[c] = car;
                     }
+                    h3 = h2;
+                    h2 = h1;
+                    h1 = d;
+                    if (kCarried) {
+                        g3 = g2;
+                        g2 = g1;
+                        g1 = car;
+                    }
+                    if (band >= 0) {
+                        out[size_t(t) * 32] = d;
+                        if (kCarried) outC[size_t(t) * 32] = car;
+                    }
                 }
-                h3 = h2;
-                h2 = h1;
-                h1 = d;
-                if (kCarried) {
-                    g3 = g2;
-                    g2 = g1;
-                    g1 = car;
-                }
-                if (band >= 0) {
-                    out[size_t(t) * 32 + lane] = d;
-                    if (kCarried) outC[size_t(t) * 32 + lane] = car;
-                }
+                __syncwarp();
             }
-            }
-            __syncwarp();
         }
         // Backward, bands bottom up over the tile's rows and the halo below; lane 0 is a band's
         // lowest row.
-        for (int c = lane; c < ww; c += 32) {
-            rowF[c] = inf;
-            if (kCarried) rowC[c] = 0.0f;
-        }
-        __syncwarp();
+        clear_rows();
         for (int band = bandsBelow - 1; band >= 0; --band) {
             const int row = r0 + 32 * band + 31 - lane;
-            const bool active = row < rw1;
-            const size_t rowBits = size_t(active ? row : r0) * p.pitch;
+            active = row < rw1;
+            rowBits = size_t(active ? row : r0) * p.pitch;
             float h1 = inf, h2 = inf, h3 = inf;
             float g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
-            uint32_t word = 0, next = 0, unknownBits = 0;
-            const int last = cw1 - 1;
-            if (active) {
-                word = p.bits[rowBits + uint32_t(last >> 5)];
-                next = (last >> 5) > 0 ? p.bits[rowBits + uint32_t(last >> 5) - 1] : 0u;
-            }
-            const float* in = store + size_t(band) * steps * 32;
-            const float* inC = storeC + size_t(band) * steps * 32;
+            uint32_t unknownBits = 0;
+            stage();
+            const float* in0 = store + size_t(band) * steps * 32 + 31 - lane;
+            const float* inC = storeC + size_t(band) * steps * 32 + 31 - lane;
             const bool tileRow = active && row < tr1;
-            // The forward values of a group's steps are loaded a group ahead (they come from L2).
+            const bool rowInside = row >= kBorderPosts && row + kBorderPosts < int(p.h);
+            // Step t is the forward pass's step ww + 61 - t. Its values of a group's steps are
+            // loaded a group ahead (they come from L2).
             float cur[kGroup], curC[kGroup];
+            auto fetch = [&](int t0) {
 #pragma unroll
-            for (int u = 0; u < kGroup; ++u) {
-                const size_t at = size_t(ww + 61 - u) * 32 + uint32_t(31 - lane);
-                cur[u] = u < steps ? in[at] : inf;
-                if (kCarried) curC[u] = u < steps ? inC[at] : 0.0f;
-            }
+                for (int u = 0; u < kGroup; ++u) {
+                    const int t = ww + 61 - t0 - u;
+                    cur[u] = t >= 0 ? in0[size_t(t) * 32] : inf;
+                    if (kCarried) curC[u] = t >= 0 ? inC[size_t(t) * 32] : 0.0f;
+                }
+            };
+            fetch(0);
             for (int t0 = 0; t0 < steps; t0 += kGroup) {
-            float nxt[kGroup], nxtC[kGroup];
+                float now[kGroup], nowC[kGroup];
 #pragma unroll
-            for (int u = 0; u < kGroup; ++u) {
-                const int t = t0 + kGroup + u;
-                const size_t at = size_t(ww + 61 - t) * 32 + uint32_t(31 - lane);
-                nxt[u] = t < steps ? in[at] : inf;
-                if (kCarried) nxtC[u] = t < steps ? inC[at] : 0.0f;
-            }
-            // Lane 0's row below over the group's columns ww - t0 down to ww - t0 - kGroup - 1
-            // (lane 31 writes only columns right of them meanwhile).
-            float below[kGroup + 2], belowC[kGroup + 2];
-            if (lane == 0) {
+                for (int u = 0; u < kGroup; ++u) {
+                    now[u] = cur[u];
+                    if (kCarried) nowC[u] = curC[u];
+                }
+                fetch(t0 + kGroup);
+                // Lane 0's row below over the group's columns ww - t0 down to
+                // ww - t0 - kGroup - 1 (lane 31 writes only columns right of them meanwhile).
+                float below[kGroup + 2], belowC[kGroup + 2];
+                bool has[kGroup];
 #pragma unroll
                 for (int i = 0; i < kGroup + 2; ++i) {
                     const int col = ww - t0 - i;
-                    const bool ok = col >= 0 && col < ww;
+                    const bool ok = lane == 0 && col >= 0 && col < ww;
                     below[i] = ok ? rowF[col] : inf;
                     if (kCarried) belowC[i] = ok ? rowC[col] : 0.0f;
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < kGroup; ++u) {
-                const int t = t0 + u;
-                if (t >= steps) {
-                    break;
+                for (int u = 0; u < kGroup; ++u) {
+                    has[u] = has_data(cw0 + ww - 1 - t0 - u + 2 * lane);
                 }
-                const int c = ww - 1 - t + 2 * lane;
-                float dL = __shfl_up_sync(0xffffffffu, h1, 1);
-                float dD = __shfl_up_sync(0xffffffffu, h2, 1);
-                float dR = __shfl_up_sync(0xffffffffu, h3, 1);
-                float eL = 0.0f, eD = 0.0f, eR = 0.0f;
-                if (kCarried) {
-                    eL = __shfl_up_sync(0xffffffffu, g1, 1);
-                    eD = __shfl_up_sync(0xffffffffu, g2, 1);
-                    eR = __shfl_up_sync(0xffffffffu, g3, 1);
-                }
-                if (lane == 0) {
-                    dR = below[u];
-                    dD = below[u + 1];
-                    dL = below[u + 2];
+#pragma unroll
+                for (int u = 0; u < kGroup; ++u) {
+                    const int c = ww - 1 - t0 - u + 2 * lane;
+                    float dL = __shfl_up_sync(0xffffffffu, h1, 1);
+                    float dD = __shfl_up_sync(0xffffffffu, h2, 1);
+                    float dR = __shfl_up_sync(0xffffffffu, h3, 1);
+                    float eL = 0.0f, eD = 0.0f, eR = 0.0f;
                     if (kCarried) {
-                        eR = belowC[u];
-                        eD = belowC[u + 1];
-                        eL = belowC[u + 2];
+                        eL = __shfl_up_sync(0xffffffffu, g1, 1);
+                        eD = __shfl_up_sync(0xffffffffu, g2, 1);
+                        eR = __shfl_up_sync(0xffffffffu, g3, 1);
                     }
-                }
-                float d = inf, car = 0.0f;
-                if (active && c >= 0 && c < ww) {
-                    const int x = cw0 + c;
-                    if ((x & 31) == 31 && c < ww - 1) {
-                        word = next;
-                        next = (x >> 5) > 0 ? p.bits[rowBits + uint32_t(x >> 5) - 1] : 0u;
+                    dR = lane == 0 ? below[u] : dR;
+                    dD = lane == 0 ? below[u + 1] : dD;
+                    dL = lane == 0 ? below[u + 2] : dL;
+                    if (kCarried) {
+                        eR = lane == 0 ? belowC[u] : eR;
+                        eD = lane == 0 ? belowC[u + 1] : eD;
+                        eL = lane == 0 ? belowC[u + 2] : eL;
                     }
-                    d = cur[u];
-                    if (kCarried) car = curC[u];
-                    const bool has = (word >> (x & 31)) & 1u;
-                    if (!has) {
-                        float s = h1 + p.dx;
-                        if (s < d) {
-                            d = s;
-                            car = g1;
-                        }
-                        s = dD + p.dy;
-                        if (s < d) {
-                            d = s;
-                            car = eD;
-                        }
-                        s = dR + p.diagonal;
-                        if (s < d) {
-                            d = s;
-                            car = eR;
-                        }
-                        s = dL + p.diagonal;
-                        if (s < d) {
-                            d = s;
-                            car = eL;
-                        }
-                    }
-                    if (lane == 31) {
+                    const bool in = active && c >= 0 && c < ww;
+                    float d = now[u], car = kCarried ? nowC[u] : 0.0f;
+                    relax(d, car, h1, g1, p.dx);
+                    relax(d, car, dD, eD, p.dy);
+                    relax(d, car, dR, eR, p.diagonal);
+                    relax(d, car, dL, eL, p.diagonal);
+                    d = !in ? inf : has[u] ? 0.0f : d;
+                    if (kCarried) car = !in ? 0.0f : has[u] ? nowC[u] : car;
+                    if (in && lane == 31) {
                         rowF[c] = d;
                         if (kCarried) rowC[c] = car;
                     }
-                    if (tileRow && x >= c0 && x < tc1) {
-                        if (p.unknown != nullptr) {
-                            const bool inside = x >= kBorderPosts && x + kBorderPosts < int(p.w) &&
-                                                row >= kBorderPosts &&
-                                                row + kBorderPosts < int(p.h);
-                            if (!has && inside && double(d) <= p.reach) {
-                                unknownBits |= 1u << (x & 31);
-                            }
-                            if ((x & 31) == 0) {
-                                p.unknown[rowBits + uint32_t(x >> 5)] = unknownBits;
-                                unknownBits = 0;
-                            }
-                        } else if (!has && double(d) < p.width) {
-                            const double u = double(d) / p.width;
-                            const double weight = 1.0 - u * u * (3.0 - 2.0 * u);
-                            p.feather[size_t(row) * p.w + uint32_t(x)] =
-                                float(weight * double(car));
+                    const int x = cw0 + c;
+                    const bool mine = in && tileRow && x >= c0 && x < tc1;
+                    if (!kCarried) {
+                        const bool unknown = mine && !has[u] && rowInside && x >= kBorderPosts &&
+                                             x + kBorderPosts < int(p.w) && double(d) <= p.reach;
+                        unknownBits |= unknown ? 1u << (x & 31) : 0u;
+                        if (mine && (x & 31) == 0) {
+                            p.unknown[rowBits + uint32_t(x >> 5)] = unknownBits;
+                            unknownBits = 0;
                         }
+                    } else if (mine && !has[u] && double(d) < p.width) {
+                        const double share = double(d) / p.width;
+                        const double weight = 1.0 - share * share * (3.0 - 2.0 * share);
+                        p.feather[size_t(row) * p.w + uint32_t(x)] = float(weight * double(car));
+                    }
+                    h3 = h2;
+                    h2 = h1;
+                    h1 = d;
+                    if (kCarried) {
+                        g3 = g2;
+                        g2 = g1;
+                        g1 = car;
                     }
                 }
-                h3 = h2;
-                h2 = h1;
-                h1 = d;
-                if (kCarried) {
-                    g3 = g2;
-                    g2 = g1;
-                    g1 = car;
-                }
+                __syncwarp();
             }
-#pragma unroll
-            for (int u = 0; u < kGroup; ++u) {
-                cur[u] = nxt[u];
-                if (kCarried) curC[u] = nxtC[u];
-            }
-            }
-            __syncwarp();
         }
     }
 }
@@ -1864,10 +1841,14 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
         const int carriedCopies = feather ? 2 : 1;
         p.rowFloats = int(std::min<size_t>(size_t(ts) + 2 * size_t(mx), width));
         const size_t bandsBelow = (std::min<size_t>(size_t(ts) + my, height) + 31) / 32;
-        p.scratchFloats = size_t(carriedCopies) * bandsBelow * (size_t(p.rowFloats) + 62) * 32;
+        p.scratchFloats = size_t(carriedCopies) * bandsBelow *
+                          ((size_t(p.rowFloats) + 62 + kGroup - 1) / kGroup * kGroup) * 32;
         const size_t rowBytes = size_t(p.rowFloats) * 4 * carriedCopies;
-        const bool sharedRows = rowBytes * kDistanceWarps <= kRowSharedBytes;
-        const size_t shared = sharedRows ? rowBytes * kDistanceWarps : 0;
+        // A window's columns lie in at most this many words.
+        p.stageWords = p.rowFloats / 32 + 2;
+        const size_t stagedBytes = rowBytes + size_t(p.stageWords) * 128;
+        const bool sharedRows = stagedBytes * kDistanceWarps <= kRowSharedBytes;
+        const size_t shared = sharedRows ? stagedBytes * kDistanceWarps : 0;
         auto kernel = feather ? (sharedRows ? distance_warp_kernel<true, true>
                                             : distance_warp_kernel<true, false>)
                               : (sharedRows ? distance_warp_kernel<false, true>
