@@ -1049,11 +1049,16 @@ struct __align__(16) LeanCrater {
     uint16_t tileX0, tileX1, tileY0, tileY1;  // the reference tiles its footprint window touches
     float cull;            // no cell beyond this distance (m) can be within its reach
     float invRadius;       // 1 / radius
-    uint32_t pad[2];
+    float invWall;         // complex craters: 1 / (1 - floorShare)
+    float invPeakBase;     // and 1 / peakBase
 };
 static_assert(sizeof(LeanCrater) == 208, "LeanCrater must be a multiple of 16 bytes");
 static_assert(offsetof(LeanCrater, harmonics) % 16 == 0 && kLeanHarmonics == 11,
               "the harmonics are read as five float4 and one float2");
+static_assert(offsetof(LeanCrater, diameter) % 16 == 0 && offsetof(LeanCrater, freshRim) % 16 == 0 &&
+                  offsetof(LeanCrater, floorShare) % 16 == 0 &&
+                  offsetof(LeanCrater, headingCos) % 16 == 0 && offsetof(LeanCrater, cull) % 16 == 0,
+              "the fields are read by float4");
 
 // The lean form of record `c` under kernel `k` (harmonics from `data`), with its footprint's
 // reference-tile box (x0, x1, y0, y1) and cull distance from the binning's count pass.
@@ -1094,6 +1099,8 @@ __device__ inline LeanCrater lean_crater(const CraterShapeKernel& k, const Crate
         l.peakHeight = size.height;
         const State s{c.freshDepth, c.freshRim, c.currentDepth, c.currentRim};
         l.kept = kept_depth(s);
+        l.invWall = 1.0f / (1.0f - l.floorShare);
+        l.invPeakBase = 1.0f / l.peakBase;
         if (c.peakCount > 0u) {
             flags |= kLeanMassifs;
             PeakSize scaled = size;
@@ -1142,66 +1149,127 @@ __device__ __forceinline__ LeanKernel lean_kernel(const CraterShapeKernel& k) {
     return LeanKernel{edge, 1.0f / (1.0f - edge)};
 }
 
+// The approximate reciprocal and reciprocal square root of normal numbers (one instruction each,
+// within 2 ulp).
+__device__ __forceinline__ float fast_reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float fast_rsqrt(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Two floats in a register pair and one multiply-add on both.
+__device__ __forceinline__ unsigned long long packed(float a, float b) {
+    unsigned long long p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+    return p;
+}
+__device__ __forceinline__ float2 unpacked(unsigned long long p) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned long long packed_fma(unsigned long long a,
+                                                         unsigned long long b,
+                                                         unsigned long long c) {
+    unsigned long long p;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(a), "l"(b), "l"(c));
+    return p;
+}
+
+// ft_shape, its branches as selects and its exterior's quotient by a constant's reciprocal.
+__device__ __forceinline__ float lean_ft_shape(float x, uint32_t rim, float freshRim,
+                                               float currentDepth) {
+    const float interior =
+        -0.228809953f + x * (0.227533882f + x * (0.083116795f - x * 0.039499407f));
+    const float polynomial =
+        0.188253307f + x * (-0.187050452f + x * (0.01844746f + x * 0.01505647f));
+    const float edge = rim == 0u ? 0.98f : rim == 2u ? 1.02f : 1.0f;
+    const float invSpan = rim == 0u ? 1.0f / 0.52f : rim == 2u ? 1.0f / 0.48f : 1.0f / 0.5f;
+    const float u = (x - edge) * invSpan;
+    const float exterior = polynomial * (1.0f - u * u);
+    float h = x <= edge ? interior : exterior;
+    if (rim == 2u) {
+        h = x > 0.98f && x <= 1.02f ? freshRim : h;
+    } else {
+        h = x <= 0.2f ? -0.181f : h;
+    }
+    h = smax(h, freshRim - currentDepth);
+    return x > 1.5f ? 0.0f : h;
+}
+
 // What lean crater `l` adds at (dx, dy) from its center (resolution times the shaped relief, the
-// round dome in place of massifs); `reached` is false beyond its reach. `shaped` receives the
-// profile distance (after the outline), which the massif peak reads.
+// round dome in place of massifs); `reached` is false beyond its reach.
+//
+// The kernel is bound by issuing instructions, so quotients are products by approximate
+// reciprocals or by reciprocals made once per crater, the distance and the direction come from
+// one reciprocal square root, and the harmonics are summed two floats to an instruction. Each is
+// within a few ulp of the correctly rounded operation, far inside the heights' 1e-3 m tolerance
+// and the cull radius's 1e-5 relative margin; the one quotient every pair's error follows, by the
+// outline's scale, is corrected (2.5 to 4.5e-7 of the heights' norm against 64 bits, as the
+// correctly rounded forms).
 __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
                                                    const LeanKernel& lk, const LeanCrater& l,
-                                                   float dx, float dy, bool& reached,
-                                                   float& shaped) {
+                                                   float dx, float dy, bool& reached) {
+    // The crater's fields, four to a load.
+    const float4 size = *reinterpret_cast<const float4*>(&l.diameter);  // diameter, radius,
+                                                                        // resolution, reach
+    const float4 state = *reinterpret_cast<const float4*>(&l.freshRim);  // freshRim,
+                                                        // currentDepth, currentRim, worn
+    const float4 inverse = *reinterpret_cast<const float4*>(&l.cull);  // cull, invRadius, invWall,
+                                                                       // invPeakBase
     const uint32_t flags = l.flags;
     const float d2 = dx * dx + dy * dy;
-    // The distance and the direction from one reciprocal square root; the quotients below by
-    // reciprocals made once per crater or by the fast divide. Each is within a few ulp of the
-    // correctly rounded operation, far inside the heights' 1e-3 m tolerance and the cull
-    // radius's 1e-5 relative margin.
-    const float inv = d2 > 0.0f ? rsqrtf(d2) : 0.0f;
+    const bool away = d2 > 1e-30f;  // else at the center: distance 0, angle 0 (KernelAngle)
+    const float inv = away ? fast_rsqrt(d2) : 0.0f;
     float distance = d2 * inv;
     if (flags & kLeanOutline) {
         // KernelProfileDistance (craters.h:1028) with the outline's scale. The share is
         // smoothstep(distance / radius), exactly 1 from the rim out.
-        const float share =
-            (distance >= l.radius ? 1.0f : outline_share(distance * l.invRadius)) * l.worn;
-        float c1 = 1.0f, s1 = 0.0f;  // the direction; angle 0 at the center, as KernelAngle
-        if (distance > 0.0f) {
-            c1 = dx * inv;
-            s1 = dy * inv;
-        }
+        const float radii = fminf(distance * inverse.y, 1.0f);
+        const float share = radii * radii * (3.0f - 2.0f * radii) * state.w;
+        const float c1 = away ? dx * inv : 1.0f, s1 = dy * inv;
         float scale = 1.0f;
         if (flags & kLeanEllipse) {
-            const float cd = c1 * l.headingCos + s1 * l.headingSin;
-            const float sd = s1 * l.headingCos - c1 * l.headingSin;
-            const float u = cd * l.across;  // cd / along
-            const float v = sd * l.along;   // sd / across
-            scale = rsqrtf(u * u + v * v);
+            // headingCos, headingSin, along, across
+            const float4 ellipse = *reinterpret_cast<const float4*>(&l.headingCos);
+            const float cd = c1 * ellipse.x + s1 * ellipse.y;
+            const float sd = s1 * ellipse.x - c1 * ellipse.y;
+            const float u = cd * ellipse.w;  // cd / along
+            const float v = sd * ellipse.z;  // sd / across
+            scale = fast_rsqrt(u * u + v * v);
         }
         const uint32_t count = (flags >> 16) & 0xffu;
-        if (share > 0.0f && count > 0u) {
-            // w = q e^{i theta}, q = share^(1/2) (1 at full share). The harmonics past `count`
-            // are zero, so Horner's rule runs over all kLeanHarmonics slots, unrolled: leading
-            // zero terms leave the sum exactly as it is.
-            const float q = share < 1.0f ? share * rsqrtf(share) : 1.0f;
+        if (share > 1e-30f && count > 0u) {
+            // w = q e^{i theta}, q = share^(1/2), and P = sum_k H_k w^k over all kLeanHarmonics
+            // slots (those past `count` are zero) by Clenshaw's recurrence, the real and the
+            // imaginary parts of the H_k side by side: b_k = H_k + 2 Re(w) b_{k+1} - q^2 b_{k+2},
+            // P = b_0 - conj(w) b_1.
+            const float q = share < 1.0f ? share * fast_rsqrt(share) : 1.0f;
             const float wr = q * c1, wi = q * s1;
-            float pr = l.harmonics[kLeanHarmonics - 1u].x, pi = l.harmonics[kLeanHarmonics - 1u].y;
-            // Harmonics 9 down to 0, two to a 16-byte load.
-            const float4* pairs = reinterpret_cast<const float4*>(l.harmonics);
+            const unsigned long long twice = packed(2.0f * wr, 2.0f * wr);
+            const unsigned long long minus = packed(-share, -share);
+            const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(l.harmonics);
+            unsigned long long b2 = 0ull;
+            unsigned long long b1 = *reinterpret_cast<const unsigned long long*>(
+                &l.harmonics[kLeanHarmonics - 1u]);
 #pragma unroll
-            for (int h = 4; h >= 0; --h) {
-                const float4 v = pairs[h];  // harmonics 2h (x, y) and 2h + 1 (z, w)
-                float t = pr * wr - pi * wi + v.z;
-                pi = pr * wi + pi * wr + v.w;
-                pr = t;
-                t = pr * wr - pi * wi + v.x;
-                pi = pr * wi + pi * wr + v.y;
-                pr = t;
+            for (int h = 4; h >= 0; --h) {  // harmonics 2 h + 1, then 2 h
+                const ulonglong2 v = pairs[h];
+                b2 = packed_fma(twice, b1, packed_fma(minus, b2, v.y));
+                b1 = packed_fma(twice, b2, packed_fma(minus, b1, v.x));
             }
+            const float2 f0 = unpacked(b1), f1 = unpacked(b2);  // b_0 and b_1
+            float pr = f0.x - (wr * f1.x + wi * f1.y), pi = f0.y + (wi * f1.x - wr * f1.y);
             // times w^first
             uint32_t first = (flags >> 8) & 0xffu;
             if (first == 2u) {
                 const float sr = wr * wr - wi * wi, si = 2.0f * wr * wi;  // w^2
-                const float t = pr * sr - pi * si;
-                pi = pr * si + pi * sr;
-                pr = t;
+                pr = pr * sr - pi * si;
             } else {
                 for (; first > 0u; --first) {
                     const float t = pr * wr - pi * wi;
@@ -1211,44 +1279,41 @@ __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
             }
             scale *= 1.0f + pr;
         }
-        distance = __fdividef(distance, scale);
+        // One correction step makes the quotient all but correctly rounded.
+        const float r = fast_reciprocal(scale), quotient = distance * r;
+        distance = fmaf(fmaf(-quotient, scale, distance), r, quotient);
     }
-    shaped = distance;
-    reached = distance < l.reach;
+    reached = distance < size.w;
     if (!reached) {
         return 0.0f;
     }
     float height;
     const uint32_t kind = flags & 3u;
+    const float x = distance * inverse.y;
     if (kind == kLeanComplex) {
         // ComplexProfileHeight (craters.h:479) with its per-crater constants made once.
-        const float x = distance * l.invRadius;
-        const float depth = l.currentDepth * l.diameter;
-        const float rim = l.currentRim * l.diameter;
+        const float depth = state.y * size.x;
+        const float rim = state.z * size.x;
         const CraterProfileKernel& p = k.profile;
         if (x >= 1.0f) {
-            if (x >= p.complexReachRadii) {
-                height = 0.0f;
-            } else {
-                const float fall = p.ejectaExponent == 3.0f ? __frcp_rn(x * x * x)
-                                                            : powf(x, -p.ejectaExponent);
-                height = rim * (fall - lk.edge) * lk.fallScale;
-            }
+            const float fall = p.ejectaExponent == 3.0f ? fast_reciprocal(x * x * x)
+                                                        : powf(x, -p.ejectaExponent);
+            height = x >= p.complexReachRadii ? 0.0f : rim * (fall - lk.edge) * lk.fallScale;
         } else {
-            height = rim - depth;
-            if (x > l.floorShare) {
-                const float t = (x - l.floorShare) / (1.0f - l.floorShare);
-                height += depth * t * t;
-            }
-            height += l.kept * peak_dome(PeakSize{l.peakHeight, l.peakBase}, distance);
+            // floorShare, peakBase, peakHeight, kept
+            const float4 peak = *reinterpret_cast<const float4*>(&l.floorShare);
+            const float t = fmaxf((x - peak.x) * inverse.z, 0.0f);
+            const float base = distance * inverse.w;
+            const float u = 1.0f - base * base;
+            const float dome = distance < peak.y ? peak.z * u * u : 0.0f;
+            height = rim - depth + depth * t * t + peak.w * dome;
         }
     } else if (kind == 1u) {
-        height = mpd_height(distance, l.diameter, l.freshRim, l.currentDepth, l.currentRim);
+        height = mpd_height(distance, size.x, state.x, state.y, state.z);
     } else {
-        height = ft_shape(distance * l.invRadius, k.profile.rim, l.freshRim, l.currentDepth) *
-                 l.diameter;
+        height = lean_ft_shape(x, k.profile.rim, state.x, state.y) * size.x;
     }
-    return l.resolution * height;
+    return size.z * height;
 }
 
 // The extras pass's contribution of crater `c` at (dx, dy): with kLeanHeavy its whole

@@ -595,35 +595,69 @@ struct LeanStager {
         phase[s] ^= 1u;
         return true;
     }
-
-    __device__ void refill(uint32_t c, uint32_t warp, uint32_t lane) {
-        if (c + 2 < chunks) {
-            __syncthreads();
-            if (warp == 0) {
-                issue(c + 2, lane);
-            }
-        }
-    }
 };
 
+constexpr uint32_t kStarts = 64;  // the power of two the search for a chunk's crater spans
+
+// A staged crater's cells of a bin: columns [c0, c0 + wide) by rows from r0, every one whose
+// center can lie within its cull radius. `inverse` is 1 / wide.
+struct LeanBox {
+    uint16_t c0, r0, wide, cells;
+    float inverse;
+};
+
+// The box, in the bin's cells, of the cell centers within `cull` of the crater, from the split
+// position of the bin's first cell center. The slack covers the rounding of the float quotients
+// (a few 1e-7 of them), so the box holds every cell the exact test per cell accepts.
+__device__ __forceinline__ LeanBox lean_box(const crater::LeanCrater& l, float x0h, float x0l,
+                                            float y0h, float y0l, float invW, float invH,
+                                            uint32_t columns, uint32_t rows) {
+    LeanBox box{0, 0, 0, 0, 0.0f};
+    const float u = crater::split_difference(l.x, l.xLow, x0h, x0l) * invW;
+    const float v = crater::split_difference(l.y, l.yLow, y0h, y0l) * invH;
+    const float ru = l.cull * fabsf(invW), rv = l.cull * fabsf(invH);
+    const float su = 0.01f + 1e-6f * (fabsf(u) + ru), sv = 0.01f + 1e-6f * (fabsf(v) + rv);
+    const int c0 = int(fminf(fmaxf(ceilf(u - ru - su), 0.0f), 32.0f));
+    const int c1 = int(fminf(fmaxf(floorf(u + ru + su) + 1.0f, 0.0f), float(columns)));
+    const int r0 = int(fminf(fmaxf(ceilf(v - rv - sv), 0.0f), 32.0f));
+    const int r1 = int(fminf(fmaxf(floorf(v + rv + sv) + 1.0f, 0.0f), float(rows)));
+    if (c0 < c1 && r0 < r1) {
+        box.c0 = uint16_t(c0);
+        box.r0 = uint16_t(r0);
+        box.wide = uint16_t(c1 - c0);
+        box.cells = uint16_t((c1 - c0) * (r1 - r0));
+        box.inverse = 1.0f / float(c1 - c0);
+    }
+    return box;
+}
+
 // The lean binned kernel (plain kernel options): each pair through `lean_contribution`; heavy
-// craters and massif peaks are left to the extras pass. Four CTAs of 256 threads per SM (64
-// registers, no spills; three CTAs at 71 registers were 7 % slower).
+// craters and massif peaks are left to the extras pass.
+//
+// Most craters are a few cells wide, so finding pairs cost as much as shaping them: testing every
+// warp's cells against every staged crater and queueing the pairs, as the general kernel does,
+// took 611 thread instructions a pair (4097^2 cells of 0.5 m, 200,000 craters of D^-2 on
+// [1, 500] m: 442 us; 358 a pair with complex craters, 818 us). Here the cells of all staged
+// craters' boxes are numbered in one sequence (a scan of the boxes' sizes), the block's threads
+// take them in turn, and 87 % of the lanes that shape a pair have one: 224 instructions for 32
+// cells of the sequence, of which four of five are pairs (about 305 and 600 us). It issues on 72 %
+// of cycles. Accumulation as above, in the block's accumulators. Four CTAs of 256 threads per SM
+// (64 registers); five with spills are no faster.
 __global__ void __launch_bounds__(kShapeThreads, 4)
-    crater_lean_shape_kernel(const CraterShapeKernel k, const CraterRecord* __restrict__ records,
-                             const float* __restrict__ data,
-                             const crater::LeanCrater* __restrict__ leans, const Grid grid,
-                             const NoData nodata, const CraterBins bins,
+    crater_lean_shape_kernel(const CraterShapeKernel k, const crater::LeanCrater* __restrict__ leans,
+                             const Grid grid, const NoData nodata, const CraterBins bins,
                              float* __restrict__ heights, uint32_t* __restrict__ flags,
                              const uint32_t polls) {
     __shared__ __align__(128) crater::LeanCrater stage[2][kLeanChunk];
     __shared__ __align__(8) uint64_t bars[2];
-    __shared__ long long accs[kShapeThreads / 32][128];
-    __shared__ uint16_t queues[kShapeThreads / 32][kQueue];
-    __shared__ float2 columns[kShapeThreads / 32][32];
-    __shared__ float2 rows[kShapeThreads / 32][4];
-    __shared__ WarpBox boxes[kShapeThreads / 32];
-    __shared__ uint8_t warpMasks[2][kLeanChunk];  // per staged crater: the warps it can touch
+    __shared__ long long acc[kBinCells * kBinCells];
+    __shared__ float2 columns[kBinCells], rows[kBinCells];
+    __shared__ uint32_t liveRows[kBinCells];  // per row, the cells that take craters
+    __shared__ LeanBox boxes[kLeanChunk];
+    __shared__ uint32_t starts[kStarts + 1];  // past the chunk: its total
+    static_assert(kLeanChunk % 32u == 0u && kLeanChunk <= kStarts && kBinCells == 32 &&
+                      kShapeThreads == 256,
+                  "the scan's shape");
 
     const uint32_t bin = bins.firstBin + blockIdx.x;
     const uint32_t binX = bin % bins.binsX, binY = bin / bins.binsX;
@@ -639,42 +673,30 @@ __global__ void __launch_bounds__(kShapeThreads, 4)
         st.start(lane);
     }
     const WarpCells w = warp_cells(grid, nodata, heights, binX, binY, warp, lane);
-    long long* acc = accs[warp];
-    uint16_t* queue = queues[warp];
+    const uint32_t cell0 = (warp * 4u + lane / 8u) * kBinCells + (lane % 8u) * kCellsPerThread;
+    uint32_t live = 0;
 #pragma unroll
     for (int j = 0; j < kCellsPerThread; ++j) {
-        acc[w.cell0 + j] = 0;
-        if (lane < 8u) {
-            columns[warp][(lane % 8u) * kCellsPerThread + j] = make_float2(w.pxh[j], w.pxl[j]);
+        acc[cell0 + j] = 0;
+        live |= w.live[j] ? 1u << ((lane % 8u) * kCellsPerThread + j) : 0u;
+        if (tid < 8u) {
+            columns[lane * kCellsPerThread + j] = make_float2(w.pxh[j], w.pxl[j]);
         }
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {  // the row's 8 lanes
+        live |= __shfl_xor_sync(0xffffffffu, live, d);
     }
     if (lane % 8u == 0u) {
-        rows[warp][lane / 8u] = make_float2(w.pyh, w.pyl);
+        rows[warp * 4u + lane / 8u] = make_float2(w.pyh, w.pyl);
+        liveRows[warp * 4u + lane / 8u] = live;
     }
-    if (lane == 0) {
-        boxes[warp] = warp_box(grid, binX, binY, warp);
-    }
-    const crater::LeanKernel lk = crater::lean_kernel(k);
+    const crater::LeanKernel lk =
+        k.profile.complex == 1u ? crater::lean_kernel(k) : crater::LeanKernel{0.0f, 0.0f};
+    const float invW = float(1.0 / grid.pixelWidth), invH = float(1.0 / grid.pixelHeight);
+    const uint32_t across = min(kBinCells, grid.width - binX * kBinCells);
+    const uint32_t down = min(kBinCells, grid.height - binY * kBinCells);
     __syncthreads();
-
-    auto drain = [&](const crater::LeanCrater* chunk, uint32_t from, uint32_t n) {
-        if (lane < n) {
-            const uint32_t code = queue[from + lane];
-            const crater::LeanCrater& l = chunk[code >> 7];
-            const uint32_t cell = code & 127u;
-            const float2 cx = columns[warp][cell & 31u];
-            const float2 cy = rows[warp][cell >> 5];
-            const float4 center = *reinterpret_cast<const float4*>(&l.x);  // x, xLow, y, yLow
-            const float dy = crater::split_difference(cy.x, cy.y, center.z, center.w);
-            const float dx = crater::split_difference(cx.x, cx.y, center.x, center.y);
-            bool reached;
-            float shaped;
-            const float v = crater::lean_contribution(k, lk, l, dx, dy, reached, shaped);
-            if (reached) {
-                add_fixed(acc + cell, to_fixed(v));
-            }
-        }
-    };
 
     uint32_t evaluated = 0;
     for (uint32_t c = 0; c < st.chunks; ++c) {
@@ -683,56 +705,89 @@ __global__ void __launch_bounds__(kShapeThreads, 4)
         }
         const uint32_t s = c & 1u;
         const uint32_t n = min(kLeanChunk, count - c * kLeanChunk);
-        // Which warps' cell boxes each staged crater's cull circle meets, one thread a crater
-        // (heavy craters are the extras pass's: none). The masks are double-buffered like the
-        // stage: the wait before chunk c + 2 is a block barrier, so chunk c's are read by then.
-        if (tid < n) {
-            const crater::LeanCrater& l = stage[s][tid];
-            uint32_t mask = 0;
-            if (!(l.flags & crater::kLeanHeavy)) {
+        // Warp 0: each crater's box and the scan of their sizes, a few neighbors a lane.
+        if (warp == 0) {
+            constexpr uint32_t kEach = kLeanChunk / 32u;
+            uint32_t size[kEach], sum = 0;
 #pragma unroll
-                for (uint32_t v = 0; v < kShapeThreads / 32; ++v) {
-                    if (!box_misses(boxes[v], l.x, l.xLow, l.y, l.yLow, l.cull)) {
-                        mask |= 1u << v;
-                    }
+            for (uint32_t i = 0; i < kEach; ++i) {
+                const uint32_t e = kEach * lane + i;
+                LeanBox box{0, 0, 0, 0, 0.0f};
+                if (e < n && !(stage[s][e].flags & crater::kLeanHeavy)) {
+                    box = lean_box(stage[s][e], columns[0].x, columns[0].y, rows[0].x, rows[0].y,
+                                   invW, invH, across, down);
                 }
+                boxes[e] = box;
+                size[i] = box.cells;
+                sum += box.cells;
             }
-            warpMasks[s][tid] = uint8_t(mask);
+            uint32_t before = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, before, d);
+                before += lane >= uint32_t(d) ? v : 0u;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, before, 31);
+            before -= sum;
+#pragma unroll
+            for (uint32_t i = 0; i < kEach; ++i) {
+                starts[kEach * lane + i] = before;
+                before += size[i];
+            }
+            for (uint32_t e = kLeanChunk + lane; e <= kStarts; e += 32u) {
+                starts[e] = total;
+            }
         }
         __syncthreads();
-        uint32_t queued = 0;  // warp-uniform
-        for (uint32_t e = 0; e < n; ++e) {
+        // Each warp takes a stretch of the numbered cells, 32 at a time: the lanes' cells stay side
+        // by side (mostly one crater's), and a lane finds its crater by search only once.
+        const uint32_t total = starts[kStarts];
+        const uint32_t stretch = (total + kShapeThreads - 1u) / kShapeThreads * 32u;
+        const uint32_t end = min((warp + 1u) * stretch, total);
+        uint32_t f = warp * stretch + lane, e = 0;
+#pragma unroll
+        for (uint32_t step = kStarts / 2; step > 0; step >>= 1) {
+            e += starts[e + step] <= f ? step : 0u;  // the last whose first cell is at or before f
+        }
+        LeanBox box = boxes[e];
+        uint32_t local = f - starts[e];
+        for (; f < end; f += 32u, local += 32u) {
+            while (local >= box.cells) {
+                local -= box.cells;
+                box = boxes[++e];
+            }
+            const uint32_t r = uint32_t((float(local) + 0.5f) * box.inverse);
+            const uint32_t row = box.r0 + r, col = box.c0 + local - r * box.wide;
+            const crater::LeanCrater& l = stage[s][e];
+            const float4 center = *reinterpret_cast<const float4*>(&l.x);  // x, xLow, y, yLow
+            const float2 cx = columns[col], cy = rows[row];
+            const float dx = crater::split_difference(cx.x, cx.y, center.x, center.y);
+            const float dy = crater::split_difference(cy.x, cy.y, center.z, center.w);
             // A lean crater is never stretched, so every cell within its cull radius lies inside
             // its footprint window: no tile test.
-            if (((warpMasks[s][e] >> warp) & 1u) == 0u) {
-                continue;  // warp-uniform
-            }
-            const crater::LeanCrater& l = stage[s][e];
-            const uint32_t need = need_mask(w, true, l.x, l.xLow, l.y, l.yLow, l.cull);
-            if (!__any_sync(0xffffffffu, need != 0u)) {
+            if (!(dx * dx + dy * dy < l.cull * l.cull) || !((liveRows[row] >> col) & 1u)) {
                 continue;
             }
-            evaluated += __popc(need);
-            queued += enqueue(queue, queued, need, e, w.cell0, lane);
-            __syncwarp();
-            while (queued >= 32u) {
-                queued -= 32u;
-                drain(stage[s], queued, 32u);
-                __syncwarp();
+            ++evaluated;
+            bool reached;
+            const float v = crater::lean_contribution(k, lk, l, dx, dy, reached);
+            if (reached) {
+                add_fixed(acc + row * kBinCells + col, to_fixed(v));
             }
         }
-        if (queued > 0u) {
-            drain(stage[s], 0u, queued);
-            __syncwarp();
+        if (c + 2 < st.chunks) {
+            __syncthreads();  // every thread has read the buffer before it is refilled
+            if (warp == 0) {
+                st.issue(c + 2, lane);
+            }
         }
-        st.refill(c, warp, lane);
     }
     const uint32_t warpPairs = __reduce_add_sync(0xffffffffu, evaluated);
     if (lane == 0 && warpPairs > 0) {
         atomicAdd(reinterpret_cast<unsigned long long*>(flags + 1), (unsigned long long)warpPairs);
     }
-    __syncwarp();
-    write_cells(grid, w, acc, heights);
+    __syncthreads();
+    write_cells(grid, w, acc + warp * 128u, heights);
 }
 
 // The extras pass after the lean kernel: heavy craters (tables, marks, terraces, shifts,
@@ -1068,7 +1123,7 @@ cudaError_t launch_crater_shape(const CraterShapeKernel& k, const CraterRecord* 
     if (leans != nullptr) {
         const auto* lean = static_cast<const crater::LeanCrater*>(leans);
         crater_lean_shape_kernel<<<nbins, kShapeThreads, 0, stream>>>(
-            k, records, data, lean, grid, nodata, strip, heights, bins.total + 1, polls);
+            k, lean, grid, nodata, strip, heights, bins.total + 1, polls);
         if (extras) {
             const cudaError_t err = cudaGetLastError();
             if (err != cudaSuccess) {
