@@ -156,7 +156,7 @@ __device__ __forceinline__ float simplex_corner(uint32_t ci, uint32_t cj, float 
                                                 uint32_t seed) {
     const float t = 0.5f - dx * dx - dy * dy;
     const float t2 = t * t;
-    const float c = t2 * t2 * gradient2(corner2(ci, cj, seed), dx, dy);
+    const float c = t2 * t2 * gradient_dot(gradient_of(corner2(ci, cj, seed)), dx, dy);
     return !(t <= 0.0f) ? c : 0.0f;
 }
 
@@ -206,12 +206,12 @@ struct WorleyD {
     float f1, f2, value;
 };
 
-__device__ __forceinline__ WorleyD worley2(float x, float y, uint32_t seed) {
-    const Cell2 c = split2(x, y);
+// The nearest feature points among the cells within `reach` cells, row by row.
+__device__ __forceinline__ WorleyD worley2_within(const Cell2& c, uint32_t seed, int32_t reach) {
     float d1 = 1e30f, d2 = 1e30f;
     uint32_t nearest = 0u;
-    for (int32_t dy = -2; dy <= 2; ++dy) {
-        for (int32_t dx = -2; dx <= 2; ++dx) {
+    for (int32_t dy = -reach; dy <= reach; ++dy) {
+        for (int32_t dx = -reach; dx <= reach; ++dx) {
             const U3 h = pcg3d(U3{uint32_t(c.ix + dx), uint32_t(c.iy + dy), seed});
             const float px = float(dx) + unit(h.y) - c.fx;
             const float py = float(dy) + unit(h.z) - c.fy;
@@ -225,7 +225,20 @@ __device__ __forceinline__ WorleyD worley2(float x, float y, uint32_t seed) {
             }
         }
     }
-    return WorleyD{sqrtf(d1), sqrtf(d2), 2.0f * unit(nearest) - 1.0f};
+    return WorleyD{d1, d2, 2.0f * unit(nearest) - 1.0f};
+}
+
+// The 5 x 5 cells' nearest points; without `second` only the nearest is read. A point two cells
+// away is at least 1 away along an axis, in the rounded arithmetic too (each operation rounds
+// monotonically), so when the 3 x 3 cells hold what is read below 1 the outer ring changes nothing
+// and is left out: 9 hashes for nearly every point instead of 25.
+__device__ __forceinline__ WorleyD worley2(float x, float y, uint32_t seed, bool second) {
+    const Cell2 c = split2(x, y);
+    WorleyD w = worley2_within(c, seed, 1);
+    if (!((second ? w.f2 : w.f1) < 1.0f)) {
+        w = worley2_within(c, seed, 2);
+    }
+    return WorleyD{sqrtf(w.f1), sqrtf(w.f2), w.value};
 }
 
 // --- 3D Perlin, for the crater texture's radial streaks (perlin.h:40-60,113-128) -----------
@@ -266,15 +279,15 @@ __device__ __forceinline__ float basis2(uint32_t basis, float x, float y, uint32
     case kBasisValue:
         return value2(x, y, seed);
     case kBasisWorleyF1:
-        return 2.0f * smin(worley2(x, y, seed).f1 * kInvSqrt2, 1.0f) - 1.0f;
+        return 2.0f * smin(worley2(x, y, seed, false).f1 * kInvSqrt2, 1.0f) - 1.0f;
     case kBasisWorleyF2:
-        return 2.0f * smin(worley2(x, y, seed).f2 * kInvSqrt5, 1.0f) - 1.0f;
+        return 2.0f * smin(worley2(x, y, seed, true).f2 * kInvSqrt5, 1.0f) - 1.0f;
     case kBasisWorleyF2MinusF1: {
-        const WorleyD d = worley2(x, y, seed);
+        const WorleyD d = worley2(x, y, seed, true);
         return 2.0f * smin((d.f2 - d.f1) * kInvSqrt5, 1.0f) - 1.0f;
     }
     case kBasisVoronoi:
-        return worley2(x, y, seed).value;
+        return worley2(x, y, seed, false).value;
     default:
         return perlin2(x, y, seed);
     }
@@ -413,90 +426,23 @@ __device__ __forceinline__ float perlin_fbm3_float(float x, float y, float z, ui
     return finish(s, kTypeFbm, 1.0f, 1.0f);
 }
 
-// Perlin fBm specialisation of `fractal2`: the same operations in the same order, without the
-// per-octave basis and type dispatch.
-__device__ __forceinline__ float perlin_fbm2(float x, float y, uint32_t seed, float wavelength,
-                                             float amplitude, int octaves, float lacunarity,
-                                             float gain) {
-    float frequency = 1.0f / wavelength;
-    float tc = 1.0f, ts = 0.0f;
-    float weight = 1.0f, sum = 0.0f, total = 0.0f;
-    for (int o = 0; o < octaves; ++o) {
-        const Octave k = octave_key(seed, o);
-        const float rx = x * tc - y * ts;
-        const float ry = x * ts + y * tc;
-        const float n = perlin2(rx * frequency + k.ox, ry * frequency + k.oy, k.seed);
-        sum += weight * n;
-        total += weight;
-        weight *= gain;
-        frequency *= lacunarity;
-        const float nc = tc * TGB_TURN_COS - ts * TGB_TURN_SIN;
-        ts = ts * TGB_TURN_COS + tc * TGB_TURN_SIN;
-        tc = nc;
-    }
-    return amplitude * sum / total;
-}
-
-__device__ __forceinline__ FractalParams params_of(const Fractal& f) {  // fractals.h:80
-    return FractalParams{f.seed, f.wavelength, f.amplitude, f.octaves, f.lacunarity,
-                         f.gain, f.basis, f.type, f.offset};
-}
-
 // Salt mixed into a fractal's seed for its warp fields (fractals.h:115).
 #define TGB_WARP_SALT 0x5bd1e995u
 
-// A fractal's value in [-1, 1], warped when it has a warp amplitude (fractals.h:151).
-__device__ __forceinline__ float evaluate_fractal(float x, float y, const Fractal& f) {
-    FractalParams unitp = params_of(f);
-    unitp.amplitude = 1.0f;
-    if (f.warpAmplitude > 0.0f) {
-        FractalParams warp{pcg(f.seed ^ TGB_WARP_SALT), f.warpWavelength, f.warpAmplitude, 4, 2.0f,
-                           0.5f, kBasisPerlin, kTypeFbm, 1.0f};
-        const float dx = fractal2(x, y, warp);
-        warp.seed = pcg(warp.seed);
-        const float dy = fractal2(x, y, warp);
-        return fractal2(x + dx, y + dy, unitp);
+// A stack's height with one more fractal of value `value` blended onto it (fractals.h:203-262).
+__device__ __forceinline__ float blend_stack(float height, float value, float amplitude,
+                                             uint32_t blend) {
+    const float scaled = amplitude * value;
+    switch (blend) {
+    case kBlendMax:
+        return smax(height, scaled);
+    case kBlendMin:
+        return smin(height, scaled);
+    case kBlendMask:
+        return height * (0.5f * (value + 1.0f));
+    default:
+        return height + scaled;
     }
-    if (f.basis == kBasisPerlin && f.type == kTypeFbm) {
-        return perlin_fbm2(x, y, f.seed, f.wavelength, 1.0f, f.octaves, f.lacunarity, f.gain);
-    }
-    return fractal2(x, y, unitp);
-}
-
-// Height of a stack of fractals: the first enabled one sets it, later ones blend
-// (fractals.h:203-262).
-__device__ __forceinline__ float evaluate_stack(float x, float y, const Fractal* fractals,
-                                                uint32_t count) {
-    float height = 0.0f;
-    bool started = false;
-    for (uint32_t i = 0; i < count; ++i) {
-        const Fractal& f = fractals[i];
-        if (!f.enabled) {
-            continue;
-        }
-        const float value = evaluate_fractal(x, y, f);
-        const float scaled = f.amplitude * value;
-        if (!started) {
-            height = scaled;
-            started = true;
-            continue;
-        }
-        switch (f.blend) {
-        case kBlendMax:
-            height = smax(height, scaled);
-            break;
-        case kBlendMin:
-            height = smin(height, scaled);
-            break;
-        case kBlendMask:
-            height *= 0.5f * (value + 1.0f);
-            break;
-        default:
-            height += scaled;
-            break;
-        }
-    }
-    return height;
 }
 
 // --- 3D noise on a body (the reference runs it only on the CPU) ---------------------------------
@@ -671,102 +617,6 @@ __device__ __forceinline__ float basis3(uint32_t basis, const Cell3& c, uint32_t
     default:
         return perlin3_cell(c, seed);
     }
-}
-
-// The golden-angle turn about (1, 2, 3) / sqrt(14) in double (Fractal3, fractal.h:286-289).
-__device__ __constant__ const double kTurn3d[3][3] = {
-    {-0.6132711010727254, -0.293401570821183, 0.7333580809050306},
-    {0.7897926788435601, -0.24097777005594262, 0.5640542870894418},
-    {0.011228581128535142, 0.9251190369776896, 0.37951111497202883}};
-
-// Fractal3 (fractal.h:284-316): world coordinates in double, each octave's lattice point split
-// in double before narrowing.
-__device__ __forceinline__ float fractal3(double x, double y, double z, const FractalParams& p) {
-    double frequency = 1.0 / double(p.wavelength);
-    double t[3][3] = {{1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}, {0.0, 0.0, 1.0}};
-    Sums s = sums_start();
-    for (int o = 0; o < p.octaves; ++o) {
-        const U3 h = pcg3d(U3{p.seed, uint32_t(o), 0u});
-        const U3 g = pcg3d(U3{p.seed, uint32_t(o), 1u});
-        const double rx = t[0][0] * x + t[0][1] * y + t[0][2] * z;
-        const double ry = t[1][0] * x + t[1][1] * y + t[1][2] * z;
-        const double rz = t[2][0] * x + t[2][1] * y + t[2][2] * z;
-        const double px = rx * frequency + double(unit(h.y));
-        const double py = ry * frequency + double(unit(h.z));
-        const double pz = rz * frequency + double(unit(g.x));
-        const float n = basis3(p.basis, split3_precise(px, py, pz), h.x);
-        s = add_octave(s, p.type, p.gain, p.offset, o, n);
-        frequency *= double(p.lacunarity);
-        double next[3][3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                next[r][c] = kTurn3d[r][0] * t[0][c] + kTurn3d[r][1] * t[1][c] +
-                             kTurn3d[r][2] * t[2][c];
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                t[r][c] = next[r][c];
-            }
-        }
-    }
-    return finish(s, p.type, p.amplitude, p.offset);
-}
-
-// EvaluateFractal3 with DomainWarp3 (fractals.h:218-243).
-__device__ __forceinline__ float evaluate_fractal3(double x, double y, double z, const Fractal& f) {
-    FractalParams unitp = params_of(f);
-    unitp.amplitude = 1.0f;
-    if (f.warpAmplitude > 0.0f) {
-        FractalParams warp{pcg(f.seed ^ TGB_WARP_SALT), f.warpWavelength, f.warpAmplitude, 4, 2.0f,
-                           0.5f, kBasisPerlin, kTypeFbm, 1.0f};
-        const double dx = double(fractal3(x, y, z, warp));
-        warp.seed = pcg(warp.seed);
-        const double dy = double(fractal3(x, y, z, warp));
-        warp.seed = pcg(warp.seed);
-        const double dz = double(fractal3(x, y, z, warp));
-        return fractal3(x + dx, y + dy, z + dz, unitp);
-    }
-    return fractal3(x, y, z, unitp);
-}
-
-// EvaluateFractals3 (fractals.h:262): the stack at a point of a body, blended as in 2D.
-__device__ __forceinline__ float evaluate_stack3(double x, double y, double z,
-                                                 const Fractal* fractals, uint32_t count) {
-    float height = 0.0f;
-    bool started = false;
-    for (uint32_t i = 0; i < count; ++i) {
-        const Fractal& f = fractals[i];
-        if (!f.enabled) {
-            continue;
-        }
-        const float value = evaluate_fractal3(x, y, z, f);
-        const float scaled = f.amplitude * value;
-        if (!started) {
-            height = scaled;
-            started = true;
-            continue;
-        }
-        switch (f.blend) {
-        case kBlendMax:
-            height = smax(height, scaled);
-            break;
-        case kBlendMin:
-            height = smin(height, scaled);
-            break;
-        case kBlendMask:
-            height *= 0.5f * (value + 1.0f);
-            break;
-        default:
-            height += scaled;
-            break;
-        }
-    }
-    return height;
 }
 
 }  // namespace noise
