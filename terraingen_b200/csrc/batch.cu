@@ -27,6 +27,7 @@
 #include "ds_tile.cuh"
 #include "kernels.h"
 #include "noise_math.cuh"
+#include "packed.cuh"
 
 namespace tgb {
 namespace {
@@ -582,6 +583,172 @@ __device__ __forceinline__ void indexed_points(const CraterShapeKernel& k,
     heights[t.heightOffset + i] = float(acc);
 }
 
+// --- the source's lattice tables ------------------------------------------------------------
+//
+// As in noise.cu, each octave of a bin whose lattice points are few reads its corners' gradients
+// from a table the CTA hashes once, kept in the features' staging buffers until they are staged.
+// Positions are monotone in the column and the row (one multiply-add each), so the bin's corner
+// cells bound them exactly.
+constexpr uint32_t kSourcePoints = 2 * kStageBytes / 12;
+
+// Octave `lane`'s table, in every warp's lane of that number: its lattice origin relative to the
+// anchor, its columns (0: not tabled), points, first point and the value that takes a cell's
+// kFloorShift bits to its place.
+struct TableBox {
+    int32_t ix0, iy0;
+    uint32_t across, points, first, base;
+    float inverse;  // 1 / across
+};
+
+__device__ __forceinline__ TableBox place_tables(const BatchNoise& noise,
+                                                 const OctaveAnchor* anchors, uint32_t c0,
+                                                 uint32_t c1, uint32_t r0, uint32_t r1) {
+    const uint32_t lane = threadIdx.x & 31u;
+    TableBox box{0, 0, 0, 0, 0, 0, 0.0f};
+    if (int(lane) < noise.octaves) {
+        const OctaveAnchor a = anchors[lane];
+        float x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float fc = float(k & 1 ? c1 : c0), fr = float(k & 2 ? r1 : r0);
+            const float qx = fmaf(fc, a.ax, fmaf(fr, a.ay, a.fx));
+            const float qy = fmaf(fc, a.bx, fmaf(fr, a.by, a.fy));
+            x0 = fminf(x0, qx);
+            x1 = fmaxf(x1, qx);
+            y0 = fminf(y0, qy);
+            y1 = fmaxf(y1, qy);
+        }
+        // Boxes within kFloorShift's range and small enough to count in 32 bits.
+        if (x0 > -2e6f && x1 < 2e6f && y0 > -2e6f && y1 < 2e6f && x1 - x0 < 1024.0f &&
+            y1 - y0 < 1024.0f) {
+            box.ix0 = __float2int_rd(x0);
+            box.iy0 = __float2int_rd(y0);
+            box.across = uint32_t(__float2int_rd(x1) - box.ix0) + 2u;
+            box.points = box.across * (uint32_t(__float2int_rd(y1) - box.iy0) + 2u);
+            box.inverse = 1.0f / float(box.across);
+        }
+    }
+    // The tables one after the other, each from a multiple of 32, while they fit.
+    const uint32_t room = (box.points + 31u) & ~31u;
+    uint32_t end = room;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t other = __shfl_up_sync(0xffffffffu, end, d);
+        end += lane >= uint32_t(d) ? other : 0u;
+    }
+    if (end > kSourcePoints) {
+        box.across = 0;
+        box.points = 0;
+    }
+    box.first = end - room;
+    box.base = box.first - (uint32_t(box.iy0) + kFloorBits) * box.across -
+               (uint32_t(box.ix0) + kFloorBits);
+    return box;
+}
+
+// Hashes the tables, 32 points of one octave to a warp's step.
+__device__ __forceinline__ void fill_tables(const BatchNoise& noise, const TableBox& box,
+                                            const OctaveAnchor* anchors, float* table) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t end =
+        __reduce_max_sync(0xffffffffu, box.points > 0u ? box.first + box.points : 0u);
+    for (uint32_t p0 = threadIdx.x & ~31u; p0 < end; p0 += blockDim.x) {
+        const uint32_t below = __ballot_sync(0xffffffffu, box.points > 0u && box.first <= p0);
+        const int o = 31 - __clz(int(below));
+        const uint32_t points = __shfl_sync(0xffffffffu, box.points, o);
+        const uint32_t across = __shfl_sync(0xffffffffu, box.across, o);
+        const uint32_t first = __shfl_sync(0xffffffffu, box.first, o);
+        const int32_t ix0 = __shfl_sync(0xffffffffu, box.ix0, o);
+        const int32_t iy0 = __shfl_sync(0xffffffffu, box.iy0, o);
+        const float inverse = __shfl_sync(0xffffffffu, box.inverse, o);
+        const uint32_t p = p0 + lane - first;
+        if (p < points) {
+            // p / across: both below 2^12, so the half keeps the float quotient off integers.
+            const uint32_t j = uint32_t((float(p) + 0.5f) * inverse);
+            const uint32_t ix = uint32_t(anchors[o].ix) + uint32_t(ix0) + p - j * across;
+            const uint32_t iy = uint32_t(anchors[o].iy) + uint32_t(iy0) + j;
+            const noise::Gradient g = noise::gradient_of(
+                corner_hash(ix * kLcgA + kLcgC, iy * kLcgA + kLcgC, noise.seedTerm[o]));
+            float* entry = table + p0 + lane;
+            entry[0] = g.x;
+            entry[kSourcePoints] = g.y;
+            entry[2 * kSourcePoints] = g.s;
+        }
+    }
+}
+
+// One tabled octave at a thread's cells, two to an instruction: perlin_at and accumulate.
+template <int kCells>
+__device__ __forceinline__ void tabled_octave(const float* table, const OctaveAnchor& a,
+                                              const BatchNoise& noise, float weight, uint32_t base,
+                                              uint32_t across, uint32_t col, uint32_t lastCol,
+                                              uint32_t row, float (&sum)[kCells],
+                                              float (&err)[kCells]) {
+    constexpr int kPairs = kCells / 2;
+    const Arithmetic on(noise.one);
+    const float fr = float(row);
+    const Pair px = both(fmaf(fr, a.ay, a.fx)), py = both(fmaf(fr, a.by, a.fy));
+    Pair fx[kPairs], fy[kPairs];
+    uint32_t cells[kPairs][2];
+    bool same = true;
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+        const Pair fc = pair_of(float(min(col + 2 * k, lastCol)),
+                                float(min(col + 2 * k + 1, lastCol)));
+        const Pair qx = fma2(fc, both(a.ax), px), qy = fma2(fc, both(a.bx), py);
+        const Pair lx = on.add_down(qx, both(kFloorShift));
+        const Pair ly = on.add_down(qy, both(kFloorShift));
+        fx[k] = on.sub(qx, on.sub(lx, both(kFloorShift)));
+        fy[k] = on.sub(qy, on.sub(ly, both(kFloorShift)));
+        float ax, bx, ay, by;
+        halves(lx, ax, bx);
+        halves(ly, ay, by);
+        cells[k][0] = base + __float_as_uint(ay) * across + __float_as_uint(ax);
+        cells[k][1] = base + __float_as_uint(by) * across + __float_as_uint(bx);
+        same = same && cells[k][0] == cells[0][0] && cells[k][1] == cells[0][0];
+    }
+    CellPair g = cell_pair<kSourcePoints>(table, cells[0][0], cells[0][1], across);
+    auto add = [&](int k) {
+        auto fade = [&](Pair t) {  // fade_fma
+            return mul2(mul2(mul2(t, t), t),
+                        fma2(t, fma2(t, both(6.0f), both(-15.0f)), both(10.0f)));
+        };
+        auto lerp = [&](Pair t, Pair p, Pair q) { return fma2(t, on.sub(q, p), p); };
+        const Pair gx = on.sub(fx[k], both(1.0f)), gy = on.sub(fy[k], both(1.0f));
+        const Pair n00 = gradient_dot2(g.g00, fx[k], fy[k]);
+        const Pair n10 = gradient_dot2(g.g10, gx, fy[k]);
+        const Pair n01 = gradient_dot2(g.g01, fx[k], gy);
+        const Pair n11 = gradient_dot2(g.g11, gx, gy);
+        const Pair u = fade(fx[k]), vv = fade(fy[k]);
+        const Pair n =
+            mul2(both(1.41421356237309505f), lerp(vv, lerp(u, n00, n10), lerp(u, n01, n11)));
+        // accumulate, its product's error taken with the sign turned.
+        const Pair before = pair_of(sum[2 * k], sum[2 * k + 1]);
+        const Pair product = mul2(both(weight), n);
+        const Pair minusError = fma2(both(-weight), n, product);
+        const Pair after = on.add(before, product);
+        const Pair bp = on.sub(after, before);
+        const Pair se = on.add(on.sub(before, on.sub(after, bp)), on.sub(product, bp));
+        const Pair total = on.add(pair_of(err[2 * k], err[2 * k + 1]), on.sub(se, minusError));
+        halves(after, sum[2 * k], sum[2 * k + 1]);
+        halves(total, err[2 * k], err[2 * k + 1]);
+    };
+    if (__all_sync(0xffffffffu, same)) {
+#pragma unroll
+        for (int k = 0; k < kPairs; ++k) {
+            add(k);
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+        if (k > 0) {
+            g = cell_pair<kSourcePoints>(table, cells[k][0], cells[k][1], across);
+        }
+        add(k);
+    }
+}
+
 template <int kBinW, int kBinH, int kCells, bool kFast>
 __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / kCells))
     batch_evaluate_kernel(const CraterShapeKernel k, const BatchNoise noise, const BatchView v) {
@@ -613,25 +780,29 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
     uint32_t phase[2] = {0u, 0u};
     uint32_t craterPairs = 0, boulderPairs = 0;
 
+    // The work queue: warp 0 holds the next bin's number, taken while the bin before was evaluated,
+    // and finds its tile, the last whose first bin is at or before it, 32 tiles to a step.
+    uint32_t upcoming = tid == 0 ? atomicAdd(&header->next, 1u) : 0u;
     for (;;) {
         __syncthreads();  // the previous bin's stage and item are no longer read
-        if (tid == 0) {
-            const uint32_t item = atomicAdd(&header->next, 1u);
+        if (tid < 32u) {
+            const uint32_t item = __shfl_sync(0xffffffffu, upcoming, 0);
             uint32_t lo = 0;
             if (item < nbins) {
-                // The last tile whose first bin is at or before the item.
-                uint32_t hi = ntiles;
-                while (hi - lo > 1u) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (v.tiles[mid].binBase <= item) {
-                        lo = mid;
-                    } else {
-                        hi = mid;
-                    }
+                for (uint32_t span = ntiles; span > 1u;) {
+                    const uint32_t step = (span + 31u) / 32u, at = lo + lane * step;
+                    const bool below = lane * step < span && v.tiles[at].binBase <= item;
+                    lo += (uint32_t(__popc(__ballot_sync(0xffffffffu, below))) - 1u) * step;
+                    span = min(step, ntiles - lo);
+                }
+                if (tid == 0) {
+                    upcoming = atomicAdd(&header->next, 1u);
                 }
             }
-            sItem = item;
-            sTile = lo;
+            if (tid == 0) {
+                sItem = item;
+                sTile = lo;
+            }
         }
         __syncthreads();
         const uint32_t item = sItem;
@@ -665,21 +836,19 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                 live[j] = row < grid.height && col0 + j < grid.width;
             }
         }
-        // Cell centers (Raster::CellCenter) or points, in double.
-        double xd[kCells], yd[kCells];
-#pragma unroll
-        for (int j = 0; j < kCells; ++j) {
+        // A cell's center (Raster::CellCenter) or the point, in double.
+        auto center = [&](int j, double& x, double& y) {
             if (points) {
                 const uint32_t i = live[j] ? first + j : 0u;
-                xd[j] = v.points[2 * (size_t(t.pointBase) + i)];
-                yd[j] = v.points[2 * (size_t(t.pointBase) + i) + 1];
+                x = v.points[2 * (size_t(t.pointBase) + i)];
+                y = v.points[2 * (size_t(t.pointBase) + i) + 1];
             } else {
-                xd[j] = grid.originX + (double(col0 + j) + 0.5) * grid.pixelWidth +
-                        (double(row) + 0.5) * grid.rowRotation;
-                yd[j] = grid.originY + (double(col0 + j) + 0.5) * grid.colRotation +
-                        (double(row) + 0.5) * grid.pixelHeight;
+                x = grid.originX + (double(col0 + j) + 0.5) * grid.pixelWidth +
+                    (double(row) + 0.5) * grid.rowRotation;
+                y = grid.originY + (double(col0 + j) + 0.5) * grid.colRotation +
+                    (double(row) + 0.5) * grid.pixelHeight;
             }
-        }
+        };
 
         // 1. The source: the base a diamond-square pass already wrote into the output, or
         //    Fractal2's octaves.
@@ -707,6 +876,18 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                 sum[j] = 0.0f;
                 err[j] = 0.0f;
             }
+            // Cells past the grid's edge take its last column and row (they are not written).
+            const uint32_t cellRow = points ? 0u : min(row, grid.height - 1u);
+            TableBox box{0, 0, 0, 0, 0, 0, 0.0f};
+            if (!points) {
+                const uint32_t bx = (local % t.binsX) * kBinW, by = (local / t.binsX) * kBinH;
+                box = place_tables(noise, v.anchors + t.anchorBase, bx,
+                                   min(bx + kBinW, grid.width) - 1u, by,
+                                   min(by + kBinH, grid.height) - 1u);
+                fill_tables(noise, box, v.anchors + t.anchorBase,
+                            reinterpret_cast<float*>(&stage[0][0]));
+                __syncthreads();
+            }
             for (int o = 0; o < noise.octaves; ++o) {
                 const uint32_t sz = noise.seedTerm[o];
                 const float w = noise.weight[o];
@@ -716,8 +897,10 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                     const double tc = noise.tc[o], ts = noise.ts[o], f = noise.frequency[o];
 #pragma unroll
                     for (int j = 0; j < kCells; ++j) {
-                        const double px = fma(fma(xd[j], tc, -yd[j] * ts), f, noise.ox[o]);
-                        const double py = fma(fma(xd[j], ts, yd[j] * tc), f, noise.oy[o]);
+                        double x, y;
+                        center(j, x, y);
+                        const double px = fma(fma(x, tc, -y * ts), f, noise.ox[o]);
+                        const double py = fma(fma(x, ts, y * tc), f, noise.oy[o]);
                         const double lx = floor(px), ly = floor(py);
                         const int32_t ix = int32_t(uint32_t(uint64_t(int64_t(lx))));
                         const int32_t iy = int32_t(uint32_t(uint64_t(int64_t(ly))));
@@ -731,8 +914,15 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                     }
                 } else {
                     const OctaveAnchor a = v.anchors[t.anchorBase + o];
+                    const uint32_t across = __shfl_sync(0xffffffffu, box.across, o);
+                    if (across != 0u) {
+                        tabled_octave<kCells>(reinterpret_cast<const float*>(&stage[0][0]), a,
+                                              noise, w, __shfl_sync(0xffffffffu, box.base, o),
+                                              across, col0, grid.width - 1u, cellRow, sum, err);
+                        continue;
+                    }
                     // Each cell from its own column, so heights do not depend on the kernel shape.
-                    const float fr = float(row);
+                    const float fr = float(cellRow);
                     const float px = fmaf(fr, a.ay, a.fx);
                     const float py = fmaf(fr, a.by, a.fy);
 #pragma unroll
@@ -757,6 +947,10 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                 h[j] = float(fma(noise.scale, double(sum[j]) + double(err[j]),
                                  double(noise.elevation)));
             }
+        }
+
+        if (!noise.baseInOutput && !points) {
+            __syncthreads();  // the stage's tables are read before features are staged there
         }
 
         // 2. Craters: each entry's data at its ref's base (the BinEntry's index field).
@@ -989,8 +1183,10 @@ __global__ void __launch_bounds__(kBinW* kBinH / kCells, 768 / (kBinW * kBinH / 
                     for (int j = 0; j < kCells; ++j) {
                         if (in[j]) {
                             ++boulderPairs;
+                            double x, y;
+                            center(j, x, y);
                             const double relief =
-                                fmax(dome(b, hypot(xd[j] - b.x, yd[j] - b.y), width), 0.0);
+                                fmax(dome(b, hypot(x - b.x, y - b.y), width), 0.0);
                             if (relief > 0.0) {
                                 best[j] = fmax(best[j], fma(b.weight, relief, double(h[j])));
                             }

@@ -401,6 +401,7 @@ int make_noise(const void* fractals, uint32_t n, float elevation, BatchNoise& no
     noise.elevation = elevation;
     noise.total = 1.0f;
     noise.scale = 0.0;
+    noise.one = 1.0f;
     const Fractal* only = nullptr;
     for (uint32_t i = 0; i < n; ++i) {
         const Fractal* f = static_cast<const Fractal*>(fractals) + i;

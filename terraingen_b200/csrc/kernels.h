@@ -313,6 +313,7 @@ struct BatchNoise {
     int32_t octaves;
     float amplitude, total, elevation;
     uint32_t baseInOutput;  // 1: the source is already in the output (a diamond-square pass)
+    float one;              // 1, as a factor the compiler does not know (packed.cuh)
     double scale;  // amplitude / total
     uint32_t seedTerm[kBatchMaxOctaves];  // octave seed through pcg3d's first LCG step
     float weight[kBatchMaxOctaves];

@@ -12,6 +12,7 @@
 
 #include "kernels.h"
 #include "noise_math.cuh"
+#include "packed.cuh"
 
 namespace tgb {
 namespace {
@@ -93,74 +94,6 @@ __device__ __forceinline__ noise::Gradient corner_gradient(uint32_t ix, uint32_t
                                                            uint32_t seedTerm) {
     return noise::gradient_of(
         corner_from_terms(ix * kLcgA + kLcgC, iy * kLcgA + kLcgC, seedTerm));
-}
-
-// Adding 1.5 * 2^23 rounding down leaves floor(q) in the low bits of a float's significand, exact
-// for |q| < 2^22: the lattice cell as an integer and, subtracting it again, as a float, without
-// the conversion unit.
-constexpr float kFloorShift = 12582912.0f;
-constexpr uint32_t kFloorBits = 0x4b400000u;
-
-// Two floats (two rows of a column) in a register pair, each operation one instruction on both
-// with the same rounding as the scalar one.
-struct Pair {
-    unsigned long long v;
-};
-__device__ __forceinline__ Pair pair_of(float a, float b) {
-    Pair p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
-    return p;
-}
-__device__ __forceinline__ void halves(Pair p, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
-}
-__device__ __forceinline__ Pair both(float a) {
-    return pair_of(a, a);
-}
-__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
-    Pair p;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
-    return p;
-}
-__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
-    Pair p;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return p;
-}
-// Sums and differences as a 1 + b and b (-1) + a, which round as a + b and a - b do: the
-// assembler fuses a packed product into a packed add (it leaves scalar ones alone under
-// -fmad=false), but not into a multiply-add. `one` is a kernel argument, so it stays a factor.
-struct Arithmetic {
-    Pair one, minusOne;
-    __device__ __forceinline__ explicit Arithmetic(float o) : one(both(o)), minusOne(both(-o)) {}
-    __device__ __forceinline__ Pair add(Pair a, Pair b) const { return fma2(a, one, b); }
-    __device__ __forceinline__ Pair sub(Pair a, Pair b) const { return fma2(b, minusOne, a); }
-    __device__ __forceinline__ Pair add_down(Pair a, Pair b) const {
-        Pair p;
-        asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(one.v), "l"(b.v));
-        return p;
-    }
-    __device__ __forceinline__ Pair fade(Pair t) const {  // noise::fade
-        const Pair inner =
-            add(mul2(t, sub(mul2(t, both(6.0f)), both(15.0f))), both(10.0f));
-        return mul2(mul2(mul2(t, t), t), inner);
-    }
-    __device__ __forceinline__ Pair lerp(Pair t, Pair a, Pair b) const {  // noise::lerp
-        return add(mul2(t, sub(b, a)), a);
-    }
-};
-
-// The gradients of one lattice corner of two rows' cells.
-struct GradientPair {
-    Pair x, y, s;
-};
-__device__ __forceinline__ Pair gradient_dot2(const GradientPair& g, Pair x, Pair y) {
-    return mul2(fma2(g.x, x, mul2(g.y, y)), g.s);  // noise::gradient_dot
-}
-__device__ __forceinline__ GradientPair gradient_pair(const float* table, uint32_t a, uint32_t b) {
-    return GradientPair{pair_of(table[a], table[b]),
-                        pair_of(table[kTablePoints + a], table[kTablePoints + b]),
-                        pair_of(table[2 * kTablePoints + a], table[2 * kTablePoints + b])};
 }
 
 // PerlinNoise2 (perlin.h:72-98) at fraction (fx, fy) of a cell, its corners' gradients given.
@@ -284,25 +217,18 @@ __global__ void __launch_bounds__(kBlockX* kBlockY, 3)
                 cells[k][1] = base + __float_as_uint(by) * across + __float_as_uint(bx);
                 same = same && cells[k][0] == cells[0][0] && cells[k][1] == cells[0][0];
             }
-            GradientPair g00, g10, g01, g11;
-            auto load = [&](uint32_t a, uint32_t b) {
-                g00 = gradient_pair(table, a, b);
-                g10 = gradient_pair(table, a + 1u, b + 1u);
-                g01 = gradient_pair(table, a + across, b + across);
-                g11 = gradient_pair(table, a + across + 1u, b + across + 1u);
-            };
+            CellPair g = cell_pair<kTablePoints>(table, cells[0][0], cells[0][1], across);
             auto add = [&](int k) {
                 const Pair gx = on.sub(fx[k], both(1.0f)), gy = on.sub(fy[k], both(1.0f));
-                const Pair n00 = gradient_dot2(g00, fx[k], fy[k]);
-                const Pair n10 = gradient_dot2(g10, gx, fy[k]);
-                const Pair n01 = gradient_dot2(g01, fx[k], gy);
-                const Pair n11 = gradient_dot2(g11, gx, gy);
+                const Pair n00 = gradient_dot2(g.g00, fx[k], fy[k]);
+                const Pair n10 = gradient_dot2(g.g10, gx, fy[k]);
+                const Pair n01 = gradient_dot2(g.g01, fx[k], gy);
+                const Pair n11 = gradient_dot2(g.g11, gx, gy);
                 const Pair u = on.fade(fx[k]), v = on.fade(fy[k]);
                 const Pair n = mul2(both(1.41421356237309505f),
                                     on.lerp(v, on.lerp(u, n00, n10), on.lerp(u, n01, n11)));
                 sum[k] = on.add(mul2(both(w), n), sum[k]);
             };
-            load(cells[0][0], cells[0][1]);
             if (__all_sync(0xffffffffu, same)) {
                 // Every lane's rows in one cell (broad octaves): no branch between the pairs.
 #pragma unroll
@@ -314,7 +240,7 @@ __global__ void __launch_bounds__(kBlockX* kBlockY, 3)
 #pragma unroll
             for (int k = 0; k < kPairs; ++k) {
                 if (k > 0) {
-                    load(cells[k][0], cells[k][1]);
+                    g = cell_pair<kTablePoints>(table, cells[k][0], cells[k][1], across);
                 }
                 add(k);
             }
