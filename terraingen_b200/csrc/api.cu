@@ -219,7 +219,12 @@ int tg_open(int ordinal, tg_device** device) {
         err = cudaMallocHost(&d->pinnedStatus, 16 * sizeof(uint32_t));
     }
     if (err == cudaSuccess) {
-        err = cudaStreamCreateWithFlags(&d->copyStream, cudaStreamNonBlocking);
+        // The side stream's small kernels go before the blocks of a large launch beside them.
+        int least = 0, greatest = 0;
+        err = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        if (err == cudaSuccess) {
+            err = cudaStreamCreateWithPriority(&d->copyStream, cudaStreamNonBlocking, greatest);
+        }
     }
     if (err == cudaSuccess) {
         err = cudaEventCreateWithFlags(&d->copied, cudaEventDisableTiming);
@@ -544,36 +549,37 @@ int crater_prepare(tg_device* d, const CraterShapeKernel& k, const CraterRecord*
     bins.binsX = (g.width + kBinCells - 1) / kBinCells;
     bins.binsY = (g.height + kBinCells - 1) / kBinCells;
     const uint32_t nbins = bins.binsX * bins.binsY;
-    TG_CUDA(d->slots[kCounts].reserve((size_t(nbins) + 1) * sizeof(uint32_t)), "allocation");
-    TG_CUDA(d->slots[kCursor].reserve(size_t(nbins) * sizeof(uint32_t)), "allocation");
+    // One zeroed run of words: each bin's cursor and extras mark, the counts (with the total
+    // after the last bin), the status behind it, on an even word for its 64-bit pairs, and the
+    // length of the extras list.
+    const size_t pad = (3 * size_t(nbins) + 1) % 2;
+    const size_t words = pad + 3 * size_t(nbins) + 1 + 4 + 1;
+    TG_CUDA(d->slots[kCounts].reserve(words * sizeof(uint32_t)), "allocation");
+    TG_CUDA(d->slots[kExtrasList].reserve(size_t(nbins) * sizeof(uint32_t)), "allocation");
     TG_CUDA(d->slots[kBoxes].reserve(size_t(n) * sizeof(int4)), "allocation");
     TG_CUDA(d->slots[kCulls].reserve(size_t(n) * sizeof(float)), "allocation");
-    TG_CUDA(d->slots[kScan].reserve(scan_scratch_words(std::max(nbins, n)) * sizeof(uint32_t)),
-            "allocation");
-    TG_CUDA(d->slots[kStatus].reserve(4 * sizeof(uint32_t)), "allocation");
-    TG_CUDA(d->slots[kPairStart].reserve((size_t(n) + 1) * sizeof(uint32_t)), "allocation");
-    TG_CUDA(d->slots[kExtrasMark].reserve(size_t(nbins) * sizeof(uint32_t)), "allocation");
-    TG_CUDA(d->slots[kExtrasList].reserve((size_t(nbins) + 1) * sizeof(uint32_t)), "allocation");
-    bins.counts = slot_ptr<uint32_t>(d, kCounts);
-    bins.cursor = slot_ptr<uint32_t>(d, kCursor);
+    TG_CUDA(d->slots[kScan].reserve(scan_scratch_words(nbins) * sizeof(uint32_t)), "allocation");
+    bins.cursor = slot_ptr<uint32_t>(d, kCounts);
+    bins.extrasMark = bins.cursor + nbins;
+    bins.counts = bins.extrasMark + nbins + pad;
+    bins.total = bins.counts + nbins + 1;
+    bins.extrasCount = bins.total + 4;
+    bins.extrasList = slot_ptr<uint32_t>(d, kExtrasList);
     bins.boxes = slot_ptr<int4>(d, kBoxes);
     bins.culls = slot_ptr<float>(d, kCulls);
-    bins.total = slot_ptr<uint32_t>(d, kStatus);
-    bins.pairStart = slot_ptr<uint32_t>(d, kPairStart);
-    bins.extrasMark = slot_ptr<uint32_t>(d, kExtrasMark);
-    bins.extrasList = slot_ptr<uint32_t>(d, kExtrasList);
-    TG_CUDA(cudaMemsetAsync(bins.counts, 0, (size_t(nbins) + 1) * sizeof(uint32_t), s), "memset");
-    TG_CUDA(cudaMemsetAsync(bins.cursor, 0, size_t(nbins) * sizeof(uint32_t), s), "memset");
-    TG_CUDA(cudaMemsetAsync(bins.total, 0, 4 * sizeof(uint32_t), s), "memset");
-    TG_CUDA(cudaMemsetAsync(bins.extrasMark, 0, size_t(nbins) * sizeof(uint32_t), s), "memset");
-    TG_CUDA(cudaMemsetAsync(bins.extrasList, 0, sizeof(uint32_t), s), "memset");
-    TG_CUDA(launch_crater_count(k, rec, n, data, foot, g, bins, slot_ptr<uint32_t>(d, kScan), s),
+    TG_CUDA(cudaMemsetAsync(bins.cursor, 0, words * sizeof(uint32_t), s), "memset");
+    const bool lean = crater_lean_entries(k);
+    if (lean) {
+        TG_CUDA(d->slots[kHarmonics].reserve(size_t(n) * kLeanCraterBytes), "allocation");
+        p.leans = d->slots[kHarmonics].ptr;
+    }
+    TG_CUDA(launch_crater_count(k, rec, n, data, foot, g, bins,
+                                lean ? d->slots[kHarmonics].ptr : nullptr, s),
             "crater count launch");
     TG_CUDA(launch_exclusive_scan(bins.counts, nbins, slot_ptr<uint32_t>(d, kScan), s),
             "scan launch");
     // The entries get the slot's capacity, at least a guess; a larger total is found on the
     // device and settled after the layer.
-    const bool lean = crater_lean_entries(k);
     p.entryBytes = lean ? kLeanEntryBytes : sizeof(BinEntry);
     const size_t guess = (lean ? 4 : 2) * size_t(n) + nbins;
     const size_t have = d->slots[kBinEntries].bytes / p.entryBytes;
@@ -581,12 +587,6 @@ int crater_prepare(tg_device* d, const CraterShapeKernel& k, const CraterRecord*
     bins.entries = slot_ptr<BinEntry>(d, kBinEntries);
     bins.capacity = uint32_t(std::min<size_t>(d->slots[kBinEntries].bytes / p.entryBytes,
                                               0xffffffffu));
-    if (lean) {
-        TG_CUDA(d->slots[kHarmonics].reserve(size_t(n) * kLeanCraterBytes), "allocation");
-        p.leans = d->slots[kHarmonics].ptr;
-        TG_CUDA(launch_crater_lean(k, rec, n, data, bins, d->slots[kHarmonics].ptr, s),
-                "lean crater launch");
-    }
     TG_CUDA(launch_crater_scatter(k, rec, n, g, bins, p.leans, s), "crater scatter launch");
     p.extras = lean;
     p.any = true;
@@ -602,11 +602,9 @@ int crater_finish(tg_device* d, const CraterPrep& p, cudaStream_t s) {
         return TG_OK;
     }
     const uint32_t nbins = p.bins.binsX * p.bins.binsY;
+    static_assert(kBoulderWords >= kCraterWords + 5, "the total and the status, side by side");
     TG_CUDA(cudaMemcpyAsync(d->pinnedStatus + kCraterWords, p.bins.counts + nbins,
-                            sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-            "copy to host");
-    TG_CUDA(cudaMemcpyAsync(d->pinnedStatus + kCraterWords + 1, p.bins.total + 1,
-                            3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
+                            5 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
             "copy to host");
     return TG_OK;
 }
@@ -679,7 +677,7 @@ int layers_settle(tg_device* d, const CraterPrep* cp, const BoulderPrep* bp, boo
     again = false;
     const uint32_t* w = d->pinnedStatus;
     if (cp != nullptr && cp->any) {
-        const uint32_t needed = w[kCraterWords], flags = w[kCraterWords + 1];
+        const uint32_t needed = w[kCraterWords], flags = w[kCraterWords + 2];
         if (flags & 1u) {
             return fail(TG_ERROR_UNSUPPORTED,
                         "craters with a datum need the ordered form (tg_craters_apply_lists)");
@@ -691,8 +689,8 @@ int layers_settle(tg_device* d, const CraterPrep* cp, const BoulderPrep* bp, boo
             if (flags & 2u) {
                 return fail(TG_ERROR_TIMEOUT, "a crater bin's staged copy did not arrive");
             }
-            d->craterPairs = (static_cast<unsigned long long>(w[kCraterWords + 3]) << 32) |
-                             w[kCraterWords + 2];
+            d->craterPairs = (static_cast<unsigned long long>(w[kCraterWords + 4]) << 32) |
+                             w[kCraterWords + 3];
         }
     }
     if (bp != nullptr && bp->any) {
@@ -1149,6 +1147,14 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
     }
     // Terrain::Fill: the source, then each layer in order (src/pipeline/terrain.cpp:299-331).
     const Positions origin{0.0, 0.0, nullptr, nullptr};
+    // The layers' binning needs no heights: it runs on the device's side stream beside the source's
+    // kernels (4097^2 cells, 200,000 craters and 1,000,000 boulders: 130 us of small kernels that
+    // leave most SMs idle), behind what the caller's stream holds already.
+    const cudaStream_t side = d->copyStream;
+    if (memory == TG_MEMORY_DEVICE) {
+        TG_CUDA(cudaEventRecord(d->copied, s), "event");
+        TG_CUDA(cudaStreamWaitEvent(side, d->copied, 0), "event wait");
+    }
     auto sources = [&]() -> int {
         TG_CUDA(launch_noise(source, g, origin, true, t->elevation, NoData{0u, 0.0f}, dh, s),
                 "noise source launch");
@@ -1158,12 +1164,17 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
         }
         return TG_OK;
     };
-    if (int st = sources()) {
-        return st;
+    const bool layers = t->n_craters > 0 || t->n_boulders > 0;
+    // Host memory: the source's kernels first, as pageable inputs hold the host while they are
+    // copied (on the side stream, beside the source). Device memory: the binning first, so that
+    // its kernels' blocks are not queued behind the source's.
+    const bool sourceFirst = memory == TG_MEMORY_HOST || !layers;
+    if (sourceFirst) {
+        if (int st = sources()) {
+            return st;
+        }
     }
-    // Host-memory layer inputs are copied on the device's copy stream while the source's
-    // kernels run; the layers wait for them.
-    const cudaStream_t on = memory == TG_MEMORY_HOST ? d->copyStream : nullptr;
+    const cudaStream_t on = memory == TG_MEMORY_HOST ? side : nullptr;
     const void *drec = nullptr, *ddata = nullptr, *dfoot = nullptr, *db = nullptr;
     if (t->n_craters > 0) {
         if (int st = stage_in(d, memory, kRecords, t->crater_records,
@@ -1188,11 +1199,6 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
             return st;
         }
     }
-    if (memory == TG_MEMORY_HOST) {
-        TG_CUDA(cudaEventRecord(d->copied, d->copyStream), "event");
-        TG_CUDA(cudaStreamWaitEvent(s, d->copied, 0), "event wait");
-    }
-    const bool layers = t->n_craters > 0 || t->n_boulders > 0;
     if (!layers) {
         return copy_heights_back(d, memory, heights, dh, cells);
     }
@@ -1204,27 +1210,33 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
         return st;
     };
     for (int attempt = 0; attempt < 2; ++attempt) {
-        if (attempt > 0) {
-            if (int st = sources()) {
-                return st;
-            }
-        }
         CraterPrep cp;
         BoulderPrep bp;
         if (t->n_craters > 0) {
             if (int st = crater_prepare(d, k, static_cast<const CraterRecord*>(drec),
                                         t->n_craters, static_cast<const float*>(ddata),
                                         t->n_crater_data, static_cast<const double*>(dfoot), g,
-                                        s, cp)) {
-                return st;
+                                        side, cp)) {
+                return drain(st);
             }
         }
         if (t->n_boulders > 0) {
             if (int st = boulder_prepare(d, static_cast<const BoulderRecord*>(db),
-                                         t->n_boulders, t->boulder_width, g, s, kBoulderCounts,
+                                         t->n_boulders, t->boulder_width, g, side, kBoulderCounts,
                                          kBoulderCursor, kBoulderStatus, bp)) {
-                return st;
+                return drain(st);
             }
+        }
+        if (!sourceFirst || attempt > 0) {
+            if (int st = sources()) {
+                return drain(st);
+            }
+        }
+        if (cudaError_t e = cudaEventRecord(d->copied, side)) {
+            return drain(cuda_fail(e, "event"));
+        }
+        if (cudaError_t e = cudaStreamWaitEvent(s, d->copied, 0)) {
+            return drain(cuda_fail(e, "event wait"));
         }
         // Host memory: the layers by strips of bin rows, each strip copied out on the copy
         // stream while the next is shaped and baked. Device memory: one launch per layer.

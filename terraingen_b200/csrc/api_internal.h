@@ -88,8 +88,6 @@ enum Slot {
     kBoulderCounts,
     kBoulderCursor,
     kBoulderStatus,
-    kPairStart,
-    kExtrasMark,
     kExtrasList,
     kRecordCraters,  // the device record builder's plan: craters, then extras
     kRecordCounts,   // its records and floats per crater, then their scans

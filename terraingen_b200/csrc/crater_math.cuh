@@ -1149,36 +1149,22 @@ __device__ __forceinline__ LeanKernel lean_kernel(const CraterShapeKernel& k) {
     return LeanKernel{edge, 1.0f / (1.0f - edge)};
 }
 
-// The approximate reciprocal and reciprocal square root of normal numbers (one instruction each,
-// within 2 ulp).
+// The approximate reciprocal of a normal number (one instruction, within 1 ulp).
 __device__ __forceinline__ float fast_reciprocal(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+// rsqrtf and __fdividef of normal numbers, the same bits without their handling of denormals.
 __device__ __forceinline__ float fast_rsqrt(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-
-// Two floats in a register pair and one multiply-add on both.
-__device__ __forceinline__ unsigned long long packed(float a, float b) {
-    unsigned long long p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
-    return p;
-}
-__device__ __forceinline__ float2 unpacked(unsigned long long p) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ unsigned long long packed_fma(unsigned long long a,
-                                                         unsigned long long b,
-                                                         unsigned long long c) {
-    unsigned long long p;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(a), "l"(b), "l"(c));
-    return p;
+__device__ __forceinline__ float fast_divide(float x, float y) {
+    float r;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
 }
 
 // ft_shape, its branches as selects and its exterior's quotient by a constant's reciprocal.
@@ -1205,13 +1191,11 @@ __device__ __forceinline__ float lean_ft_shape(float x, uint32_t rim, float fres
 // What lean crater `l` adds at (dx, dy) from its center (resolution times the shaped relief, the
 // round dome in place of massifs); `reached` is false beyond its reach.
 //
-// The kernel is bound by issuing instructions, so quotients are products by approximate
-// reciprocals or by reciprocals made once per crater, the distance and the direction come from
-// one reciprocal square root, and the harmonics are summed two floats to an instruction. Each is
-// within a few ulp of the correctly rounded operation, far inside the heights' 1e-3 m tolerance
-// and the cull radius's 1e-5 relative margin; the one quotient every pair's error follows, by the
-// outline's scale, is corrected (2.5 to 4.5e-7 of the heights' norm against 64 bits, as the
-// correctly rounded forms).
+// The kernel is bound by issuing instructions, so the distance and the direction come from one
+// reciprocal square root, the profile's quotients are products by reciprocals, most of them made
+// once per crater, and the quotient by the outline's scale is the fast divide: each within a few
+// ulp of the correctly rounded operation, far inside the heights' 1e-3 m tolerance and the cull
+// radius's 1e-5 relative margin.
 __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
                                                    const LeanKernel& lk, const LeanCrater& l,
                                                    float dx, float dy, bool& reached) {
@@ -1229,7 +1213,7 @@ __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
     float distance = d2 * inv;
     if (flags & kLeanOutline) {
         // KernelProfileDistance (craters.h:1028) with the outline's scale. The share is
-        // smoothstep(distance / radius), exactly 1 from the rim out.
+        // smoothstep(distance / radius).
         const float radii = fminf(distance * inverse.y, 1.0f);
         const float share = radii * radii * (3.0f - 2.0f * radii) * state.w;
         const float c1 = away ? dx * inv : 1.0f, s1 = dy * inv;
@@ -1245,31 +1229,31 @@ __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
         }
         const uint32_t count = (flags >> 16) & 0xffu;
         if (share > 1e-30f && count > 0u) {
-            // w = q e^{i theta}, q = share^(1/2), and P = sum_k H_k w^k over all kLeanHarmonics
-            // slots (those past `count` are zero) by Clenshaw's recurrence, the real and the
-            // imaginary parts of the H_k side by side: b_k = H_k + 2 Re(w) b_{k+1} - q^2 b_{k+2},
-            // P = b_0 - conj(w) b_1.
+            // w = q e^{i theta}, q = share^(1/2) (1 at full share). The harmonics past `count`
+            // are zero, so Horner's rule runs over all kLeanHarmonics slots, unrolled: leading
+            // zero terms leave the sum exactly as it is.
             const float q = share < 1.0f ? share * fast_rsqrt(share) : 1.0f;
             const float wr = q * c1, wi = q * s1;
-            const unsigned long long twice = packed(2.0f * wr, 2.0f * wr);
-            const unsigned long long minus = packed(-share, -share);
-            const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(l.harmonics);
-            unsigned long long b2 = 0ull;
-            unsigned long long b1 = *reinterpret_cast<const unsigned long long*>(
-                &l.harmonics[kLeanHarmonics - 1u]);
+            float pr = l.harmonics[kLeanHarmonics - 1u].x, pi = l.harmonics[kLeanHarmonics - 1u].y;
+            // Harmonics 9 down to 0, two to a 16-byte load.
+            const float4* pairs = reinterpret_cast<const float4*>(l.harmonics);
 #pragma unroll
-            for (int h = 4; h >= 0; --h) {  // harmonics 2 h + 1, then 2 h
-                const ulonglong2 v = pairs[h];
-                b2 = packed_fma(twice, b1, packed_fma(minus, b2, v.y));
-                b1 = packed_fma(twice, b2, packed_fma(minus, b1, v.x));
+            for (int h = 4; h >= 0; --h) {
+                const float4 v = pairs[h];  // harmonics 2h (x, y) and 2h + 1 (z, w)
+                float t = pr * wr - pi * wi + v.z;
+                pi = pr * wi + pi * wr + v.w;
+                pr = t;
+                t = pr * wr - pi * wi + v.x;
+                pi = pr * wi + pi * wr + v.y;
+                pr = t;
             }
-            const float2 f0 = unpacked(b1), f1 = unpacked(b2);  // b_0 and b_1
-            float pr = f0.x - (wr * f1.x + wi * f1.y), pi = f0.y + (wi * f1.x - wr * f1.y);
             // times w^first
             uint32_t first = (flags >> 8) & 0xffu;
             if (first == 2u) {
                 const float sr = wr * wr - wi * wi, si = 2.0f * wr * wi;  // w^2
-                pr = pr * sr - pi * si;
+                const float t = pr * sr - pi * si;
+                pi = pr * si + pi * sr;
+                pr = t;
             } else {
                 for (; first > 0u; --first) {
                     const float t = pr * wr - pi * wi;
@@ -1279,9 +1263,7 @@ __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
             }
             scale *= 1.0f + pr;
         }
-        // One correction step makes the quotient all but correctly rounded.
-        const float r = fast_reciprocal(scale), quotient = distance * r;
-        distance = fmaf(fmaf(-quotient, scale, distance), r, quotient);
+        distance = fast_divide(distance, scale);
     }
     reached = distance < size.w;
     if (!reached) {

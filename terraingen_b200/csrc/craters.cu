@@ -1,16 +1,17 @@
 // Crater shaping over a grid (ApplyCraters, src/layers/craters/shaping/apply.cpp:339-376).
 //
 // Plain path, in four stream-ordered launches:
-//   1. count   - one warp per crater: its footprint window on the grid, exactly as
+//   1. count   - a thread per crater: its footprint window on the grid, exactly as
 //                CratersOnRaster / PixelWindowIn compute it (apply.cpp:225-237,
 //                src/raster/cell_loops.cpp:21-28), turned into the range of the reference's
-//                16-cell tiles it touches, and one count per kBinCells-square bin it covers;
+//                16-cell tiles it touches, its lean form under plain kernel options, and one
+//                count per kBinCells-square bin it covers;
 //   2. scan    - exclusive prefix sum of the bin counts;
-//   3. scatter - one warp per crater: a 160-byte BinEntry (record + tile range) into each bin;
+//   3. scatter - a thread per crater: its index (other options: a 160-byte BinEntry, record + tile
+//                range) into each bin;
 //   4. shape   - one CTA per bin: the bin's entries are staged in shared memory by TMA bulk
-//                copies (cp.async.bulk + mbarrier, double-buffered), each warp ballots whether
-//                any of its cells needs a crater, and each thread adds the crater to its 4 cells
-//                (one 16-byte store per thread at the end).
+//                copies (cp.async.bulk + mbarrier, double-buffered) and added to its cells (one
+//                16-byte store per thread at the end).
 //
 // Coverage matches the reference's: a crater is evaluated at every cell of each 16x16 tile its
 // window touches (apply.cpp:119-143, 199-222), whatever the bin size here.
@@ -33,81 +34,124 @@ constexpr uint32_t kChunk = 96;        // entries per staged chunk (15 KB)
 
 using namespace binning;
 
-// Binning runs over (crater, bin) pairs, so a crater covering thousands of bins costs no more
-// than as many small ones: the footprint pass finds each crater's tile box, cull radius and bin
-// count; an exclusive scan of those counts numbers the pairs; the count and scatter passes take
-// one pair per thread (grid-stride), each finding its crater by binary search in the scan.
+// Binning takes a thread per crater: one of few bins goes through them itself, a block's wider
+// craters are then taken by its warps, and the widest (a 500 m one covers thousands of bins) by the
+// whole block. Numbering the (crater, bin) pairs by a scan and searching it per pair spread them
+// evenly too, at the price of the scan's three launches, a dozen dependent reads a pair and a pass
+// over the craters apart from the lean records' (kernels of 3168 craters on 513^2 cells: 45 us, and
+// of 200,000 on 4097^2: 112 us; 28 and 92 now).
+constexpr uint32_t kBinThreads = 128;
+constexpr uint32_t kOwnBins = 4, kWarpBins = 512;
+
+// The bins of a reference-tile box.
+struct BinBox {
+    uint32_t x0, y0, wide, count;
+};
+__device__ __forceinline__ BinBox bin_box(int4 tiles) {
+    constexpr uint32_t kTilesPerBin = kBinCells / kRefTileCells;
+    BinBox b{0, 0, 0, 0};
+    if (tiles.x <= tiles.y) {
+        b.x0 = uint32_t(tiles.x) / kTilesPerBin;
+        b.y0 = uint32_t(tiles.z) / kTilesPerBin;
+        b.wide = uint32_t(tiles.y) / kTilesPerBin - b.x0 + 1u;
+        b.count = b.wide * (uint32_t(tiles.w) / kTilesPerBin - b.y0 + 1u);
+    }
+    return b;
+}
+
+// The bins of `box` from the `first`th on, every `stride`th: their slots first, four at a time in
+// flight (reserve(column, row)), then what goes there (put(crater, slot, column, row)).
+template <typename Reserve, typename Put>
+__device__ __forceinline__ void take_bins(uint32_t crater, const BinBox& box, uint32_t first,
+                                          uint32_t stride, Reserve reserve, Put put) {
+    constexpr uint32_t kFlight = 4;
+    for (uint32_t i = first; i < box.count; i += kFlight * stride) {
+        uint32_t slot[kFlight], x[kFlight], y[kFlight];
+#pragma unroll
+        for (uint32_t u = 0; u < kFlight; ++u) {
+            const uint32_t at = i + u * stride;
+            const uint32_t down = at / box.wide;
+            x[u] = box.x0 + at - down * box.wide;
+            y[u] = box.y0 + down;
+            slot[u] = at < box.count ? reserve(x[u], y[u]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kFlight; ++u) {
+            if (i + u * stride < box.count) {
+                put(crater, slot[u], x[u], y[u]);
+            }
+        }
+    }
+}
+
+// take_bins for every bin of each of the block's craters (the calling thread's is `mine`, of the
+// bins `box`); every thread of the block calls it.
+template <typename Reserve, typename Put>
+__device__ __forceinline__ void for_crater_bins(uint32_t mine, const BinBox& box, Reserve reserve,
+                                                Put put) {
+    __shared__ uint32_t wideCount;
+    __shared__ uint32_t wideCraters[kBinThreads];
+    __shared__ BinBox wideBoxes[kBinThreads];
+    if (threadIdx.x == 0) {
+        wideCount = 0;
+    }
+    __syncthreads();
+    if (box.count > kOwnBins) {
+        const uint32_t at = atomicAdd(&wideCount, 1u);
+        wideCraters[at] = mine;
+        wideBoxes[at] = box;
+    } else {
+        take_bins(mine, box, 0u, 1u, reserve, put);
+    }
+    __syncthreads();
+    for (uint32_t c = threadIdx.x / 32u; c < wideCount; c += kBinThreads / 32u) {
+        if (wideBoxes[c].count <= kWarpBins) {
+            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x % 32u, 32u, reserve, put);
+        }
+    }
+    for (uint32_t c = 0; c < wideCount; ++c) {
+        if (wideBoxes[c].count > kWarpBins) {
+            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x, kBinThreads, reserve, put);
+        }
+    }
+}
 
 // Per crater: its footprint (the 16-cell tile window and cull radius, as CraterReach and
-// TileLists give it) and how many bins it covers, into pairStart[i] (scanned afterwards).
-__global__ void crater_footprint_kernel(const CraterShapeKernel k,
-                                        const CraterRecord* __restrict__ records, uint32_t n,
-                                        const float* __restrict__ data,
-                                        const double* __restrict__ footprints, const Grid grid,
-                                        CraterBins bins, uint32_t* __restrict__ flags) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) {
-        return;
-    }
-    constexpr uint32_t kTilesPerBin = kBinCells / kRefTileCells;
-    const CraterRecord& r = records[i];
-    const Footprint f = crater_footprint(k, r, data, footprints, i, grid);
-    bins.boxes[i] = f.tiles;
-    bins.culls[i] = f.cull;
-    uint32_t pairs = 0;
-    if (f.tiles.x <= f.tiles.y) {
-        pairs = (uint32_t(f.tiles.y) / kTilesPerBin - uint32_t(f.tiles.x) / kTilesPerBin + 1u) *
-                (uint32_t(f.tiles.w) / kTilesPerBin - uint32_t(f.tiles.z) / kTilesPerBin + 1u);
-        if (r.hasDatum == 1u) {
-            atomicOr(flags, 1u);
-        }
-        // Work for the extras pass after the lean kernel (heavy records, massif peaks).
-        if (crater_needs_extras(k, r) || (crater_is_complex(k, r) && r.peakCount > 0u)) {
-            atomicOr(flags, 4u);
-        }
-    }
-    bins.pairStart[i] = pairs;
-}
-
-// The crater of pair p: the last crater whose first pair is at most p (pairStart scanned, with
-// pairStart[n] the number of pairs).
-__device__ __forceinline__ uint32_t pair_crater(const uint32_t* __restrict__ start, uint32_t n,
-                                                uint32_t p) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(start + mid) <= p) {
-            lo = mid;
-        } else {
-            hi = mid;
+// TileLists give it), its LeanCrater with `leans`, and one more entry in each bin it covers.
+__global__ void __launch_bounds__(kBinThreads)
+    crater_footprint_kernel(const CraterShapeKernel k, const CraterRecord* __restrict__ records,
+                            uint32_t n, const float* __restrict__ data,
+                            const double* __restrict__ footprints, const Grid grid,
+                            CraterBins bins, crater::LeanCrater* __restrict__ leans) {
+    const uint32_t i = blockIdx.x * kBinThreads + threadIdx.x;
+    BinBox box{0, 0, 0, 0};
+    if (i < n) {
+        const CraterRecord& r = records[i];
+        const Footprint f = crater_footprint(k, r, data, footprints, i, grid);
+        bins.boxes[i] = f.tiles;
+        bins.culls[i] = f.cull;
+        box = bin_box(f.tiles);
+        if (box.count > 0u) {
+            uint32_t* flags = bins.total + 1;
+            if (r.hasDatum == 1u) {
+                atomicOr(flags, 1u);
+            }
+            // Work for the extras pass after the lean kernel (heavy records, massif peaks).
+            if (crater_needs_extras(k, r) || (crater_is_complex(k, r) && r.peakCount > 0u)) {
+                atomicOr(flags, 4u);
+            }
+            if (leans != nullptr) {
+                leans[i] = crater::lean_crater(k, r, data, i, f.tiles, f.cull);
+            }
         }
     }
-    return lo;
-}
-
-// Pair p's crater and bin.
-__device__ __forceinline__ void pair_bin(const CraterBins& bins, uint32_t n, uint32_t p,
-                                         uint32_t& crater, int4& tiles, uint32_t& bx,
-                                         uint32_t& by) {
-    constexpr uint32_t kTilesPerBin = kBinCells / kRefTileCells;
-    crater = pair_crater(bins.pairStart, n, p);
-    tiles = bins.boxes[crater];
-    const uint32_t local = p - __ldg(bins.pairStart + crater);
-    const uint32_t bx0 = uint32_t(tiles.x) / kTilesPerBin;
-    const uint32_t wide = uint32_t(tiles.y) / kTilesPerBin - bx0 + 1u;
-    bx = bx0 + local % wide;
-    by = uint32_t(tiles.z) / kTilesPerBin + local / wide;
-}
-
-__global__ void crater_bin_count_kernel(uint32_t n, CraterBins bins) {
-    const uint32_t pairs = bins.pairStart[n];
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < pairs;
-         p += gridDim.x * blockDim.x) {
-        uint32_t crater, bx, by;
-        int4 tiles;
-        pair_bin(bins, n, p, crater, tiles, bx, by);
-        atomicAdd(bins.counts + by * bins.binsX + bx, 1u);
-    }
+    for_crater_bins(
+        i, box,
+        [&](uint32_t bx, uint32_t by) {
+            atomicAdd(bins.counts + by * bins.binsX + bx, 1u);
+            return 0u;
+        },
+        [](uint32_t, uint32_t, uint32_t, uint32_t) {});
 }
 
 // Whether a massif peak of `radius` m around (x, y) can reach a cell center of bin (bx, by): the
@@ -129,28 +173,32 @@ __device__ inline bool peak_meets_bin(const Grid& g, double x, double y, double 
     return c0 <= c1 && r0 <= r1;
 }
 
-// Each pair's entry in its bin's next slot. With `leans` the entries are crater indices, with
-// kHeavyEntry where the extras pass has work (a heavy crater in all its bins, a massif peak in the
-// bins its reach meets), and each such bin is listed once in bins.extrasList; otherwise they are
-// BinEntry copies (the record and the tail).
-__global__ void crater_bin_scatter_kernel(const CraterShapeKernel k,
-                                          const CraterRecord* __restrict__ records, uint32_t n,
-                                          const crater::LeanCrater* __restrict__ leans,
-                                          const Grid grid, CraterBins bins) {
+// Each crater's entry in the next slot of every bin it covers. With `leans` the entries are crater
+// indices, with kHeavyEntry where the extras pass has work (a heavy crater in all its bins, a
+// massif peak in the bins its reach meets), and each such bin is listed once in bins.extrasList;
+// otherwise they are BinEntry copies (the record and the tail).
+__global__ void __launch_bounds__(kBinThreads)
+    crater_bin_scatter_kernel(const CraterShapeKernel k, const CraterRecord* __restrict__ records,
+                              uint32_t n, const crater::LeanCrater* __restrict__ leans,
+                              const Grid grid, CraterBins bins) {
     if (!crater_bins_usable(bins)) {
         return;
     }
-    const uint32_t pairs = bins.pairStart[n];
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < pairs;
-         p += gridDim.x * blockDim.x) {
-        uint32_t crater, bx, by;
-        int4 t;
-        pair_bin(bins, n, p, crater, t, bx, by);
+    const uint32_t mine = blockIdx.x * kBinThreads + threadIdx.x;
+    BinBox box{0, 0, 0, 0};
+    if (mine < n) {
+        box = bin_box(bins.boxes[mine]);
+    }
+    const auto reserve = [&](uint32_t bx, uint32_t by) {
         const uint32_t b = by * bins.binsX + bx;
-        const uint32_t slot = bins.counts[b] + atomicAdd(bins.cursor + b, 1u);
+        return bins.counts[b] + atomicAdd(bins.cursor + b, 1u);
+    };
+    for_crater_bins(mine, box, reserve, [&](uint32_t crater, uint32_t slot, uint32_t bx,
+                                            uint32_t by) {
         if (slot >= bins.capacity) {
-            continue;  // the total fits the capacity (checked above); never taken
+            return;  // the total fits the capacity (checked above); never taken
         }
+        const uint32_t b = by * bins.binsX + bx;
         const CraterRecord& r = records[crater];
         if (leans != nullptr) {
             bool extras = crater_needs_extras(k, r);
@@ -161,10 +209,11 @@ __global__ void crater_bin_scatter_kernel(const CraterShapeKernel k,
             }
             reinterpret_cast<uint32_t*>(bins.entries)[slot] = crater | (extras ? kHeavyEntry : 0u);
             if (extras && atomicOr(bins.extrasMark + b, 1u) == 0u) {
-                bins.extrasList[1u + atomicAdd(bins.extrasList, 1u)] = b;
+                bins.extrasList[atomicAdd(bins.extrasCount, 1u)] = b;
             }
-            continue;
+            return;
         }
+        const int4 t = bins.boxes[crater];
         const int4* src = reinterpret_cast<const int4*>(records + crater);
         int4* dst = reinterpret_cast<int4*>(bins.entries + slot);
 #pragma unroll
@@ -174,7 +223,7 @@ __global__ void crater_bin_scatter_kernel(const CraterShapeKernel k,
         dst[9] = make_int4(int(uint32_t(t.x) | (uint32_t(t.y) << 16)),
                            int(uint32_t(t.z) | (uint32_t(t.w) << 16)),
                            __float_as_int(bins.culls[crater]), int(crater));
-    }
+    });
 }
 
 // (amplitude, phase) of each record's outline harmonics as (amplitude cos phase,
@@ -525,17 +574,6 @@ __global__ void __launch_bounds__(kShapeThreads)
     write_cells(grid, w, acc, heights);
 }
 
-// Each crater's LeanCrater (crater_math.cuh), made once after the count pass.
-__global__ void crater_lean_kernel(const CraterShapeKernel k,
-                                   const CraterRecord* __restrict__ records, uint32_t n,
-                                   const float* __restrict__ data, const CraterBins bins,
-                                   crater::LeanCrater* __restrict__ leans) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        leans[i] = crater::lean_crater(k, records[i], data, i, bins.boxes[i], bins.culls[i]);
-    }
-}
-
 constexpr uint32_t kLeanChunk = 64;  // 13 KB a buffer
 
 // The lean kernel's staging: a bin holds crater indices, and warp 0 gathers each chunk's
@@ -805,10 +843,10 @@ __global__ void __launch_bounds__(kShapeThreads)
     if ((bins.total[1] & 4u) == 0u || !crater_bins_usable(bins)) {
         return;  // no heavy record nor massif peak in the layer
     }
-    const uint32_t listed = bins.extrasList[0];
+    const uint32_t listed = *bins.extrasCount;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t item = blockIdx.x; item < listed; item += gridDim.x) {
-        const uint32_t bin = bins.extrasList[1u + item];
+        const uint32_t bin = bins.extrasList[item];
         if (bin < bins.firstBin || bin >= bins.firstBin + binsInStrip) {
             continue;  // block-uniform: another strip's bin
         }
@@ -1036,26 +1074,16 @@ cudaError_t launch_exclusive_scan(uint32_t* counts, uint32_t n, uint32_t* scratc
     return cudaGetLastError();
 }
 
-// Grid of the pair-parallel passes (grid-stride over the pairs, whose number stays on the device).
-constexpr uint32_t kPairBlocks = 148u * 8u;
-
 cudaError_t launch_crater_count(const CraterShapeKernel& k, const CraterRecord* records,
                                 uint32_t n, const float* data, const double* footprints,
-                                const Grid& grid, const CraterBins& bins, uint32_t* scratch,
+                                const Grid& grid, const CraterBins& bins, void* leans,
                                 cudaStream_t stream) {
+    static_assert(sizeof(crater::LeanCrater) == kLeanCraterBytes, "lean crater size");
     if (n == 0) {
         return cudaSuccess;
     }
-    crater_footprint_kernel<<<(n + 255) / 256, 256, 0, stream>>>(k, records, n, data, footprints,
-                                                                 grid, bins, bins.total + 1);
-    cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) {
-        err = launch_exclusive_scan(bins.pairStart, n, scratch, stream);
-    }
-    if (err != cudaSuccess) {
-        return err;
-    }
-    crater_bin_count_kernel<<<kPairBlocks, 256, 0, stream>>>(n, bins);
+    crater_footprint_kernel<<<(n + kBinThreads - 1) / kBinThreads, kBinThreads, 0, stream>>>(
+        k, records, n, data, footprints, grid, bins, static_cast<crater::LeanCrater*>(leans));
     return cudaGetLastError();
 }
 
@@ -1065,20 +1093,8 @@ cudaError_t launch_crater_scatter(const CraterShapeKernel& k, const CraterRecord
     if (n == 0) {
         return cudaSuccess;
     }
-    crater_bin_scatter_kernel<<<kPairBlocks, 256, 0, stream>>>(
+    crater_bin_scatter_kernel<<<(n + kBinThreads - 1) / kBinThreads, kBinThreads, 0, stream>>>(
         k, records, n, static_cast<const crater::LeanCrater*>(leans), grid, bins);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_crater_lean(const CraterShapeKernel& k, const CraterRecord* records, uint32_t n,
-                               const float* data, const CraterBins& bins, void* leans,
-                               cudaStream_t stream) {
-    static_assert(sizeof(crater::LeanCrater) == kLeanCraterBytes, "lean crater size");
-    if (n == 0) {
-        return cudaSuccess;
-    }
-    crater_lean_kernel<<<(n + 127) / 128, 128, 0, stream>>>(
-        k, records, n, data, bins, static_cast<crater::LeanCrater*>(leans));
     return cudaGetLastError();
 }
 

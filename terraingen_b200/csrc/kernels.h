@@ -76,35 +76,28 @@ struct CraterBins {
     uint32_t* cursor;    // [bins]
     BinEntry* entries;   // [capacity]
     uint32_t capacity;
-    uint32_t* total;     // [1] entries needed
+    uint32_t* total;     // [4], zeroed: unused, flags, the pairs evaluated (64 bits, aligned)
     int4* boxes;         // [craters] reference-tile box per crater (x0, x1, y0, y1); empty: x0 > x1
     float* culls;        // [craters] cull distance per crater
     uint32_t firstBin;   // the bin of a launch's first block (a strip of bin rows)
-    uint32_t* pairStart; // [craters + 1]: bins per crater, then their exclusive scan
     uint32_t* extrasMark;  // [bins], zeroed: a bin listed for the extras pass
-    uint32_t* extrasList;  // [bins + 1], [0] zeroed: how many bins are listed, then the bins
+    uint32_t* extrasList;  // [bins]: the bins listed
+    uint32_t* extrasCount;  // [1], zeroed: how many
 };
 
-// Per crater: its footprint's reference-tile box on `grid` and the number of bins it covers,
-// added to bins.counts. `footprints` (x, y, reach in meters, as doubles) is optional; without it
-// the footprint follows from the record (center hi + lo, reach = outline stretch x reachRadii x
-// radius).
-// `scratch` holds scan_scratch_words(n) words for the scan of the pairs.
-cudaError_t launch_crater_count(const CraterShapeKernel& k, const CraterRecord* records,
-                                uint32_t n, const float* data, const double* footprints,
-                                const Grid& grid, const CraterBins& bins, uint32_t* scratch,
-                                cudaStream_t stream);
-// The plain path's lean craters (crater_math.cuh LeanCrater): kLeanCraterBytes per crater, made
-// by launch_crater_lean; with them the bins hold kLeanEntryBytes entries, else 160-byte BinEntry.
-// The plain path's lean craters (crater_math.cuh LeanCrater): kLeanCraterBytes per crater, made
-// by launch_crater_lean after the count pass (it reads the footprint boxes and culls). With them
-// the bins hold 4-byte crater indices (the shaping kernel gathers each entry's LeanCrater into
-// shared memory), else 160-byte BinEntry copies of the records.
+// The plain path's lean craters (crater_math.cuh LeanCrater): kLeanCraterBytes per crater. With
+// them the bins hold 4-byte crater indices (the shaping kernel gathers each entry's LeanCrater
+// into shared memory), else 160-byte BinEntry copies of the records.
 constexpr size_t kLeanCraterBytes = 208;
 constexpr size_t kLeanEntryBytes = 4;
-cudaError_t launch_crater_lean(const CraterShapeKernel& k, const CraterRecord* records, uint32_t n,
-                               const float* data, const CraterBins& bins, void* leans,
-                               cudaStream_t stream);
+// Per crater: its footprint's reference-tile box on `grid`, one more in bins.counts for each bin
+// it covers and, with `leans`, its lean form. `footprints` (x, y, reach in meters, as doubles) is
+// optional; without it the footprint follows from the record (center hi + lo, reach = outline
+// stretch x reachRadii x radius).
+cudaError_t launch_crater_count(const CraterShapeKernel& k, const CraterRecord* records,
+                                uint32_t n, const float* data, const double* footprints,
+                                const Grid& grid, const CraterBins& bins, void* leans,
+                                cudaStream_t stream);
 // Scatters each crater into its bins (its index when `leans` is given, else a BinEntry); an entry
 // whose crater needs the extras pass (crater_needs_extras) carries kHeavyEntry in its index.
 cudaError_t launch_crater_scatter(const CraterShapeKernel& k, const CraterRecord* records,
