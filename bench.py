@@ -51,10 +51,10 @@ NOISE_OPS_PER_CELL_OCTAVE = 180
 # cos, amplitude, kept share's pow, product, sum) 77, scale and division 2, reach test 1, profile
 # 8, resolution and the add 2: 104, plus the ellipse of 5 % of craters (10): 105.
 CRATER_OPS_PER_PAIR = 105
-# Thread instructions the lean crater kernel executes per pair, measured with ncu on this
-# workload (smsp__inst_executed x active lanes / pairs: 771.3 M x 29.79 / 64,216,893): the
-# issue-rate view of the same work (loads, the queue, compares and selects).
-CRATER_THREAD_INST_PER_PAIR = 358
+# Thread instructions the lean crater kernel executes per pair, measured with ncu on a tile of
+# this workload's make (smsp__inst_executed x active lanes / pairs: 580.1 M x 28.37 / 58,126,370):
+# the issue-rate view of the same work (loads, the boxes' cells, compares and selects).
+CRATER_THREAD_INST_PER_PAIR = 283
 # Counted from terraingen_b200/csrc/boulders.cu per (cell, boulder) pair: window test 6, offset
 # and hypot 12, dome band average (2 sqrt, 2 asin, clamps) 60, max-composite 4; FP64.
 BOULDER_OPS_PER_PAIR = 82

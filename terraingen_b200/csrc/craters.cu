@@ -676,10 +676,10 @@ __device__ __forceinline__ LeanBox lean_box(const crater::LeanCrater& l, float x
 // warp's cells against every staged crater and queueing the pairs, as the general kernel does,
 // took 611 thread instructions a pair (4097^2 cells of 0.5 m, 200,000 craters of D^-2 on
 // [1, 500] m: 442 us; 358 a pair with complex craters, 818 us). Here the cells of all staged
-// craters' boxes are numbered in one sequence (a scan of the boxes' sizes), the block's threads
-// take them in turn, and 87 % of the lanes that shape a pair have one: 224 instructions for 32
-// cells of the sequence, of which four of five are pairs (about 305 and 600 us). It issues on 72 %
-// of cycles. Accumulation as above, in the block's accumulators. Four CTAs of 256 threads per SM
+// craters' boxes are numbered in one sequence (a scan of the boxes' sizes) and the block's threads
+// take them in turn: four of five of the sequence's cells are pairs, and 87 % of the lanes that
+// shape one have one. 283 a pair with complex craters, 683 us; 331 us without. It issues on 77 % of
+// cycles. Accumulation as above, in the block's accumulators. Four CTAs of 256 threads per SM
 // (64 registers); five with spills are no faster.
 __global__ void __launch_bounds__(kShapeThreads, 4)
     crater_lean_shape_kernel(const CraterShapeKernel k, const crater::LeanCrater* __restrict__ leans,
