@@ -1151,7 +1151,8 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
     // kernels (4097^2 cells, 200,000 craters and 1,000,000 boulders: 130 us of small kernels that
     // leave most SMs idle), behind what the caller's stream holds already.
     const cudaStream_t side = d->copyStream;
-    if (memory == TG_MEMORY_DEVICE) {
+    const bool layers = t->n_craters > 0 || t->n_boulders > 0;
+    if (memory == TG_MEMORY_DEVICE && layers) {
         TG_CUDA(cudaEventRecord(d->copied, s), "event");
         TG_CUDA(cudaStreamWaitEvent(side, d->copied, 0), "event wait");
     }
@@ -1164,7 +1165,6 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
         }
         return TG_OK;
     };
-    const bool layers = t->n_craters > 0 || t->n_boulders > 0;
     // Host memory: the source's kernels first, as pageable inputs hold the host while they are
     // copied (on the side stream, beside the source). Device memory: the binning first, so that
     // its kernels' blocks are not queued behind the source's.
