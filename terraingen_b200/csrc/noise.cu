@@ -11,6 +11,7 @@
 #include <cmath>
 
 #include "kernels.h"
+#include "lattice_box.h"
 #include "noise_math.cuh"
 #include "packed.cuh"
 
@@ -301,20 +302,14 @@ void place_tables(Octaves& oct, const Grid& g, const Positions& at, uint32_t til
     if (at.xs != nullptr || at.ys != nullptr) {
         return;
     }
-    double reach = 0.0;  // the largest |x| + |y| of a cell center
-    for (int k = 0; k < 4; ++k) {
-        const double c = k & 1 ? double(g.width) : 0.0, r = k & 2 ? double(g.height) : 0.0;
-        const double x = g.originX + c * g.pixelWidth + r * g.rowRotation - at.originX;
-        const double y = g.originY + c * g.colRotation + r * g.pixelHeight - at.originY;
-        reach = std::max(reach, std::fabs(x) + std::fabs(y));
-    }
+    const double reach = lattice_reach(g, at);
     const double spanC = double(kBlockX - 1), spanR = double(tileRows - 1);
     const double wide = spanC * std::fabs(g.pixelWidth) + spanR * std::fabs(g.rowRotation);
     const double high = spanC * std::fabs(g.colRotation) + spanR * std::fabs(g.pixelHeight);
     for (int o = 0; o < oct.count; ++o) {
         const double f = std::fabs(double(oct.frequency[o]));
         const double tc = std::fabs(double(oct.tc[o])), ts = std::fabs(double(oct.ts[o]));
-        if (!(reach * f < 262144.0)) {
+        if (!lattice_tabled(reach, oct.frequency[o])) {
             continue;
         }
         // The box's cells, their far corners, the margin on each side and one for rounding.

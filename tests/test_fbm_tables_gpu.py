@@ -57,3 +57,16 @@ def test_layer_skips_nodata(device):
         outs.append(out)
     np.testing.assert_array_equal(outs[0], outs[1])
     assert (outs[0][base == -9999.0] == -9999.0).all()
+
+
+@pytest.mark.parametrize("origin", [(np.nan, 0.0), (0.0, np.nan), (np.inf, np.nan), (-np.inf, 0.0),
+                                    (1e39, 0.0)])
+def test_origins_that_are_no_floats_give_nan(device, origin):
+    """Such positions are not looked up in a table; every octave is NaN, as the fractal's sum."""
+    grid = N.Grid(65, 33, 5.0, 0.5, 0.0, -3.0, 0.0, -0.5)
+    k = noise_layer_kernel([fractal(seed=2, wavelength=64.0, amplitude=3.0, octaves=7)])
+    out = np.zeros((33, 65), np.float32)
+    N.check(device._lib.tg_noise_layer(device._handle, k.ctypes.data, k.nbytes, C.byref(grid),
+                                       *origin, out.ctypes.data, N.NoData(0, 0.0),
+                                       N.TG_MEMORY_HOST, None))
+    assert np.isnan(out).all()
