@@ -26,6 +26,7 @@
 #include "crater_math.cuh"
 #include "ds_tile.cuh"
 #include "kernels.h"
+#include "lattice_box.h"
 #include "noise_math.cuh"
 #include "packed.cuh"
 
@@ -648,25 +649,12 @@ __device__ __forceinline__ TableBox place_tables(const BatchNoise& noise,
     const uint32_t lane = threadIdx.x & 31u;
     TableBox box{0, 0, 0, 0, 0, 0, 0.0f};
     if (int(lane) < noise.octaves) {
-        const OctaveAnchor a = anchors[lane];
-        float x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float fc = float(k & 1 ? c1 : c0), fr = float(k & 2 ? r1 : r0);
-            const float qx = fmaf(fc, a.ax, fmaf(fr, a.ay, a.fx));
-            const float qy = fmaf(fc, a.bx, fmaf(fr, a.by, a.fy));
-            x0 = fminf(x0, qx);
-            x1 = fmaxf(x1, qx);
-            y0 = fminf(y0, qy);
-            y1 = fmaxf(y1, qy);
-        }
-        // Boxes within kFloorShift's range and small enough to count in 32 bits.
-        if (x0 > -2e6f && x1 < 2e6f && y0 > -2e6f && y1 < 2e6f && x1 - x0 < 1024.0f &&
-            y1 - y0 < 1024.0f) {
-            box.ix0 = __float2int_rd(x0);
-            box.iy0 = __float2int_rd(y0);
-            box.across = uint32_t(__float2int_rd(x1) - box.ix0) + 2u;
-            box.points = box.across * (uint32_t(__float2int_rd(y1) - box.iy0) + 2u);
+        const LatticeBox at = lattice_box(anchors[lane], c0, c1, r0, r1);
+        if (lattice_boxed(at)) {
+            box.ix0 = __float2int_rd(at.x0);
+            box.iy0 = __float2int_rd(at.y0);
+            box.across = uint32_t(__float2int_rd(at.x1) - box.ix0) + 2u;
+            box.points = box.across * (uint32_t(__float2int_rd(at.y1) - box.iy0) + 2u);
             box.inverse = 1.0f / float(box.across);
         }
     }
