@@ -6,6 +6,7 @@
 #pragma once
 
 #include "kernels.h"
+#include "normal_parts.h"
 
 namespace tgb {
 namespace {
@@ -36,8 +37,8 @@ __device__ __forceinline__ Words philox(Words c, uint32_t k0, uint32_t k1) {
 // its product with any |k| <= 64 is exact in float.
 constexpr float kLn2High = 0.693145751953125f;
 constexpr float kLn2Low = float(0.69314718055994530942 - 0.693145751953125);
-// pi 2^-31: a signed 32-bit integer times this is pi times the integer's share of 2^31.
-constexpr float kPiOver2p31 = float(3.14159265358979323846 / 2147483648.0);
+// pi 2^-52: a 53-bit integer times this is pi times the integer's share of 2^52.
+constexpr float kPiOver2p52 = float(3.14159265358979323846 / 4503599627370496.0);
 
 // log(1 - u) in float for u = (high 2^26 + low) 2^-53, high of 27 bits and low of 26, with relative
 // accuracy for u near 0 and near 1, one path for every lane. Below u = 1/4, log1p(f) with f = -u;
@@ -70,11 +71,10 @@ __device__ __forceinline__ float log_of_rest(uint32_t high, uint32_t low) {
 // src/random/samplers.cpp:65-69), sqrt(-2 log(1 - u1)) cos(2 pi u2). The reference evaluates it
 // in double; here in float on arguments formed from the draws' integers: the logarithm as above,
 // the square root as x rsqrt(x), and the cosine of pi a with a = 2 u2 taken modulo 2 into [-1, 1)
-// as a signed 32-bit integer (u2's bits past the 32nd are below 1e-9 of a turn; the hardware
-// cosine is within 4e-7 there). Within 1e-5 of the double normal (a few 1e-7 of the radius; under
+// (the hardware cosine is within 4e-7 there). Within 1e-5 of the double normal (a few 1e-7 of the radius; under
 // 2e-5 m in the refined heights), for the fewest instructions: the refinement is bound by issuing
 // them, and the 64-bit shifts, leading zeros and conversions of the whole 53-bit integers took 7 %
-// of its time (5121^2 cells: 868 us, 807 now; 320 or more threads a block, or 192, are slower).
+// of its time (5121^2 cells: 868 us, 818 now; 320 or more threads a block, or 192, are slower).
 __device__ __forceinline__ double node_normal(int64_t col, int64_t row, int level,
                                               uint32_t seed) {
     const uint32_t high = uint32_t((col >> 32) ^ (row >> 32));
@@ -82,8 +82,7 @@ __device__ __forceinline__ double node_normal(int64_t col, int64_t row, int leve
                            seed, kMidpointDisplacementStream);
     const float twice = -2.0f * log_of_rest(b.x >> 5u, b.y >> 6u);
     const float radius = twice > 0.0f ? twice * rsqrtf(twice) : 0.0f;
-    const int32_t turn = int32_t((b.z & ~31u) | (b.w >> 27u));
-    const float c = __cosf(float(turn) * kPiOver2p31);
+    const float c = __cosf(normal_turn(b.z, b.w) * kPiOver2p52);
     return double(radius * c);
 }
 
