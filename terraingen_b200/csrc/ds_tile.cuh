@@ -40,47 +40,38 @@ constexpr float kLn2Low = float(0.69314718055994530942 - 0.693145751953125);
 // pi 2^-52: a 53-bit integer times this is pi times the integer's share of 2^52.
 constexpr float kPiOver2p52 = float(3.14159265358979323846 / 4503599627370496.0);
 
-// log(1 - u) in float for u = (high 2^26 + low) 2^-53, high of 27 bits and low of 26, with relative
-// accuracy for u near 0 and near 1, one path for every lane. Below u = 1/4, log1p(f) with f = -u;
-// from there on 1 - u, formed from the integers' difference, is 2^k (1 + f) with 1 + f in
-// [0.75, 1.5). Either float comes from its two integers by one multiply-add, and log(1 + f) =
+// log(2^k (1 + f)) in float, 1 + f in [0.75, 1.5), one path for every lane: log(1 + f) =
 // 2 atanh(s) = 2 (s + s^3/3 + s^5/5 + s^7/7 + s^9/9 + ...) for s = f / (2 + f), |s| <= 1/5, the
 // series cut after s^9 (its tail is below 1e-8 of the sum): within 3e-7 of the logarithm relative.
-__device__ __forceinline__ float log_of_rest(uint32_t high, uint32_t low) {
-    const bool small = high < (1u << 25);
-    // 2^53 - (high 2^26 + low) = (2^27 - 1 - high) 2^26 + (2^26 - low).
-    const uint32_t h = small ? high : 0x7ffffffu - high;
-    const uint32_t l = small ? low : 0x4000000u - low;
-    const float v = fmaf(float(int32_t(h)), 0x1p-27f, float(int32_t(l)) * 0x1p-53f);
-    const int32_t bits = __float_as_int(v);
-    const int32_t k = small ? 0 : (bits - 0x3f400000) >> 23;
-    const float f = small ? -v : __int_as_float(bits - (k << 23)) - 1.0f;
+__device__ __forceinline__ float log_of_ratio(const NormalRatio& r) {
+    const float f = r.f;
     const float s = __fdividef(f, 2.0f + f);
     const float s2 = s * s;
     float series = fmaf(s2, 1.0f / 9.0f, 1.0f / 7.0f);
     series = fmaf(s2, series, 1.0f / 5.0f);
     series = fmaf(s2, series, 1.0f / 3.0f);
     const float log1p = fmaf(2.0f * s * s2, series, 2.0f * s);
-    const float kf = float(k);
-    return fmaf(kf, kLn2High, fmaf(kf, kLn2Low, log1p));
+    const float k = float(r.k);
+    return fmaf(k, kLn2High, fmaf(k, kLn2Low, log1p));
 }
 
 // The standard normal of node (col, row) of `level` (Refinement::Displacement,
 // diamond_square.cpp:382-389): one Philox block is RandomStream's first two NextDouble draws
 // (u1, u2, 53 bits each, exact), turned into a normal by Box-Muller (StandardNormal,
 // src/random/samplers.cpp:65-69), sqrt(-2 log(1 - u1)) cos(2 pi u2). The reference evaluates it
-// in double; here in float on arguments formed from the draws' integers: the logarithm as above,
-// the square root as x rsqrt(x), and the cosine of pi a with a = 2 u2 taken modulo 2 into [-1, 1)
-// (the hardware cosine is within 4e-7 there). Within 1e-5 of the double normal (a few 1e-7 of the radius; under
-// 2e-5 m in the refined heights), for the fewest instructions: the refinement is bound by issuing
-// them, and the 64-bit shifts, leading zeros and conversions of the whole 53-bit integers took 7 %
-// of its time (5121^2 cells: 868 us, 818 now; 320 or more threads a block, or 192, are slower).
+// in double; here in float on arguments formed exactly from the draws' integers and rounded once:
+// the logarithm as above, the square root as x rsqrt(x), and the cosine of pi a with a = 2 u2 taken
+// modulo 2 into [-1, 1) (the hardware cosine is within 4e-7 there). Within 1e-5 of the double normal
+// (a few 1e-7 of the radius; under 2e-5 m in the refined heights), for the fewest instructions: the
+// refinement is bound by issuing them, and the 64-bit shifts, leading zeros and compares of the
+// whole 53-bit integers, where their words do as well, took its time from 819 to 868 us (5121^2
+// cells; 320 or more threads a block, or 192, are slower).
 __device__ __forceinline__ double node_normal(int64_t col, int64_t row, int level,
                                               uint32_t seed) {
     const uint32_t high = uint32_t((col >> 32) ^ (row >> 32));
     const Words b = philox(Words{uint32_t(col), uint32_t(row), uint32_t(level) | (high << 5), 0u},
                            seed, kMidpointDisplacementStream);
-    const float twice = -2.0f * log_of_rest(b.x >> 5u, b.y >> 6u);
+    const float twice = -2.0f * log_of_ratio(normal_ratio(b.x, b.y));
     const float radius = twice > 0.0f ? twice * rsqrtf(twice) : 0.0f;
     const float c = __cosf(normal_turn(b.z, b.w) * kPiOver2p52);
     return double(radius * c);

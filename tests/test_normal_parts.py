@@ -18,6 +18,13 @@ def parts(tmp_path_factory):
 extern "C" void turns(const uint32_t* z, const uint32_t* w, int n, float* out) {
     for (int i = 0; i < n; ++i) out[i] = tgb::normal_turn(z[i], w[i]);
 }
+extern "C" void ratios(const uint32_t* x, const uint32_t* y, int n, float* f, int* k) {
+    for (int i = 0; i < n; ++i) {
+        const tgb::NormalRatio r = tgb::normal_ratio(x[i], y[i]);
+        f[i] = r.f;
+        k[i] = r.k;
+    }
+}
 """)
     return lib
 
@@ -47,3 +54,17 @@ def test_a_turn_takes_all_bits_of_its_draw(parts):
     # 53-bit integers are exact in double, so this rounds once.
     want = np.where(m >= 1 << 52, m - (1 << 53), m).astype(np.float64).astype(np.float32)
     np.testing.assert_array_equal(got, want)
+
+
+def test_a_logarithm_takes_its_argument_rounded_once(parts):
+    m, x, y = _draws()
+    f, k = np.zeros(len(m), np.float32), np.zeros(len(m), np.int32)
+    parts.ratios(*(a.ctypes.data_as(C.c_void_p) for a in (x, y)), len(m),
+                 f.ctypes.data_as(C.c_void_p), k.ctypes.data_as(C.c_void_p))
+    n = (1 << 53) - m
+    # n = 2^e (1 + f): e the exponent of n / 0.75, exactly.
+    bits = np.array([int(v).bit_length() for v in n], np.int64)
+    e = np.where((bits >= 2) & (n >= 3 * (1 << np.maximum(bits - 2, 0))), bits, bits - 1)
+    np.testing.assert_array_equal(k, e - 53)
+    want = (n - (1 << e)).astype(np.float64) * 2.0 ** -e.astype(np.float64)
+    np.testing.assert_array_equal(f, want.astype(np.float32))
