@@ -1149,12 +1149,6 @@ __device__ __forceinline__ LeanKernel lean_kernel(const CraterShapeKernel& k) {
     return LeanKernel{edge, 1.0f / (1.0f - edge)};
 }
 
-// The approximate reciprocal of a normal number (one instruction, within 1 ulp).
-__device__ __forceinline__ float fast_reciprocal(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 // rsqrtf and __fdividef of normal numbers, the same bits without their handling of denormals.
 __device__ __forceinline__ float fast_rsqrt(float x) {
     float r;
@@ -1186,6 +1180,43 @@ __device__ __forceinline__ float lean_ft_shape(float x, uint32_t rim, float fres
     }
     h = smax(h, freshRim - currentDepth);
     return x > 1.5f ? 0.0f : h;
+}
+
+// Lean crater `l`'s profile height at profile distance `distance` (the round dome in place of
+// massifs), before its resolution weight.
+__device__ __forceinline__ float lean_height(const CraterShapeKernel& k, const LeanKernel& lk,
+                                             const LeanCrater& l, float distance) {
+    // The crater's fields, four to a load.
+    const float4 size = *reinterpret_cast<const float4*>(&l.diameter);  // diameter, radius,
+                                                                        // resolution, reach
+    const float4 state = *reinterpret_cast<const float4*>(&l.freshRim);  // freshRim,
+                                                        // currentDepth, currentRim, worn
+    const float4 inverse = *reinterpret_cast<const float4*>(&l.cull);  // cull, invRadius, invWall,
+                                                                       // invPeakBase
+    const uint32_t kind = l.flags & 3u;
+    const float x = distance * inverse.y;
+    if (kind == kLeanComplex) {
+        // ComplexProfileHeight (craters.h:479) with its per-crater constants made once.
+        const float depth = state.y * size.x;
+        const float rim = state.z * size.x;
+        const CraterProfileKernel& p = k.profile;
+        if (x >= 1.0f) {
+            const float fall = p.ejectaExponent == 3.0f ? __frcp_rn(x * x * x)
+                                                        : powf(x, -p.ejectaExponent);
+            return x >= p.complexReachRadii ? 0.0f : rim * (fall - lk.edge) * lk.fallScale;
+        }
+        // floorShare, peakBase, peakHeight, kept
+        const float4 peak = *reinterpret_cast<const float4*>(&l.floorShare);
+        const float t = fmaxf((x - peak.x) * inverse.z, 0.0f);
+        const float base = distance * inverse.w;
+        const float u = 1.0f - base * base;
+        const float dome = distance < peak.y ? peak.z * u * u : 0.0f;
+        return rim - depth + depth * t * t + peak.w * dome;
+    }
+    if (kind == 1u) {
+        return mpd_height(distance, size.x, state.x, state.y, state.z);
+    }
+    return lean_ft_shape(x, k.profile.rim, state.x, state.y) * size.x;
 }
 
 // What lean crater `l` adds at (dx, dy) from its center (resolution times the shaped relief, the
@@ -1269,33 +1300,7 @@ __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
     if (!reached) {
         return 0.0f;
     }
-    float height;
-    const uint32_t kind = flags & 3u;
-    const float x = distance * inverse.y;
-    if (kind == kLeanComplex) {
-        // ComplexProfileHeight (craters.h:479) with its per-crater constants made once.
-        const float depth = state.y * size.x;
-        const float rim = state.z * size.x;
-        const CraterProfileKernel& p = k.profile;
-        if (x >= 1.0f) {
-            const float fall = p.ejectaExponent == 3.0f ? fast_reciprocal(x * x * x)
-                                                        : powf(x, -p.ejectaExponent);
-            height = x >= p.complexReachRadii ? 0.0f : rim * (fall - lk.edge) * lk.fallScale;
-        } else {
-            // floorShare, peakBase, peakHeight, kept
-            const float4 peak = *reinterpret_cast<const float4*>(&l.floorShare);
-            const float t = fmaxf((x - peak.x) * inverse.z, 0.0f);
-            const float base = distance * inverse.w;
-            const float u = 1.0f - base * base;
-            const float dome = distance < peak.y ? peak.z * u * u : 0.0f;
-            height = rim - depth + depth * t * t + peak.w * dome;
-        }
-    } else if (kind == 1u) {
-        height = mpd_height(distance, size.x, state.x, state.y, state.z);
-    } else {
-        height = lean_ft_shape(x, k.profile.rim, state.x, state.y) * size.x;
-    }
-    return size.z * height;
+    return size.z * lean_height(k, lk, l, distance);
 }
 
 // The extras pass's contribution of crater `c` at (dx, dy): with kLeanHeavy its whole
