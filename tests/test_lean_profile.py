@@ -108,3 +108,12 @@ def test_the_ejecta_falls_by_a_rounded_reciprocal(profiles):
     want = np.where(x >= np.float32(3.0), np.float32(0.0), rim * (fall - edge) * scale)
     assert want.dtype == np.float32
     np.testing.assert_array_equal(lean, want)
+
+
+def test_a_complex_wall_rises_by_a_rounded_quotient(profiles):
+    # Outside the peak, where the dome adds nothing.
+    distance = (16.0 * _radii(0.2, 1.0)).astype(np.float32)
+    lean, general, (_, _, _, floor_share, peak_base) = profiles(1, 0, 32.0, distance)
+    wall = (distance >= peak_base) & (distance < 16.0)
+    assert floor_share < 0.2 and wall.sum() > 20000
+    np.testing.assert_array_equal(lean[wall], general[wall])
