@@ -1100,7 +1100,7 @@ __device__ inline LeanCrater lean_crater(const CraterShapeKernel& k, const Crate
         const State s{c.freshDepth, c.freshRim, c.currentDepth, c.currentRim};
         l.kept = kept_depth(s);
         l.invWall = 1.0f / (1.0f - l.floorShare);
-        l.invPeakBase = 1.0f / l.peakBase;
+        l.invPeakBase = fminf(1.0f / l.peakBase, 3.402823466e38f);  // finite: 0 / base is 0
         if (c.peakCount > 0u) {
             flags |= kLeanMassifs;
             PeakSize scaled = size;
@@ -1218,7 +1218,7 @@ __device__ __forceinline__ float lean_height(const CraterShapeKernel& k, const L
         // floorShare, peakBase, peakHeight, kept
         const float4 peak = *reinterpret_cast<const float4*>(&l.floorShare);
         const float t = fmaxf(quotient_by(x - peak.x, 1.0f - peak.x, inverse.z), 0.0f);
-        const float base = distance * inverse.w;
+        const float base = quotient_by(distance, peak.y, inverse.w);
         const float u = 1.0f - base * base;
         const float dome = distance < peak.y ? peak.z * u * u : 0.0f;
         return rim - depth + depth * t * t + peak.w * dome;

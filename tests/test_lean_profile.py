@@ -117,3 +117,11 @@ def test_a_complex_wall_rises_by_a_rounded_quotient(profiles):
     wall = (distance >= peak_base) & (distance < 16.0)
     assert floor_share < 0.2 and wall.sum() > 20000
     np.testing.assert_array_equal(lean[wall], general[wall])
+
+
+def test_a_peaks_dome_falls_by_a_rounded_quotient(profiles):
+    _, _, (_, _, _, floor_share, peak_base) = profiles(1, 0, 32.0, np.zeros(1, np.float32))
+    distance = (peak_base * _radii(0.0, 1.1)).astype(np.float32)
+    lean, general, _ = profiles(1, 0, 32.0, distance)
+    assert 0.0 < peak_base < 16.0
+    np.testing.assert_array_equal(lean, general)
