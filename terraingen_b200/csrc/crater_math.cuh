@@ -1171,7 +1171,7 @@ __device__ __forceinline__ float quotient_by(float a, float b, float inverse) {
     return fmaf(fmaf(-q, b, a), inverse, q);
 }
 
-// ft_shape, its branches as selects and its exterior's quotient by a constant's reciprocal.
+// ft_shape, its branches as selects.
 __device__ __forceinline__ float lean_ft_shape(float x, uint32_t rim, float freshRim,
                                                float currentDepth) {
     const float interior =
@@ -1179,8 +1179,10 @@ __device__ __forceinline__ float lean_ft_shape(float x, uint32_t rim, float fres
     const float polynomial =
         0.188253307f + x * (-0.187050452f + x * (0.01844746f + x * 0.01505647f));
     const float edge = rim == 0u ? 0.98f : rim == 2u ? 1.02f : 1.0f;
-    const float invSpan = rim == 0u ? 1.0f / 0.52f : rim == 2u ? 1.0f / 0.48f : 1.0f / 0.5f;
-    const float u = (x - edge) * invSpan;
+    const float invSpan = rim == 0u   ? 1.0f / (1.5f - 0.98f)
+                          : rim == 2u ? 1.0f / (1.5f - 1.02f)
+                                      : 1.0f / (1.5f - 1.0f);
+    const float u = quotient_by(x - edge, 1.5f - edge, invSpan);
     const float exterior = polynomial * (1.0f - u * u);
     float h = x <= edge ? interior : exterior;
     if (rim == 2u) {

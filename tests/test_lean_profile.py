@@ -125,3 +125,13 @@ def test_a_peaks_dome_falls_by_a_rounded_quotient(profiles):
     lean, general, _ = profiles(1, 0, 32.0, distance)
     assert 0.0 < peak_base < 16.0
     np.testing.assert_array_equal(lean, general)
+
+
+@pytest.mark.parametrize("rim", [0, 1, 2])
+def test_a_simple_crater_is_the_general_profile(profiles, rim):
+    # The edges of its pieces, the floats beside them, and all between.
+    edges = np.float32([0.2, 0.98, 1.0, 1.02, 1.5])
+    x = np.concatenate([_radii(0.0, 1.6).astype(np.float32), edges,
+                        np.nextafter(edges, np.float32(0.0)), np.nextafter(edges, np.float32(2.0))])
+    lean, general, _ = profiles(0, rim, 4.0, np.float32(2.0) * x)
+    np.testing.assert_array_equal(lean, general)
