@@ -556,6 +556,7 @@ int crater_prepare(tg_device* d, const CraterShapeKernel& k, const CraterRecord*
     const size_t words = pad + 3 * size_t(nbins) + 1 + 4 + 1;
     TG_CUDA(d->slots[kCounts].reserve(words * sizeof(uint32_t)), "allocation");
     TG_CUDA(d->slots[kExtrasList].reserve(size_t(nbins) * sizeof(uint32_t)), "allocation");
+    TG_CUDA(d->slots[kWideCraters].reserve(size_t(n) * sizeof(uint32_t)), "allocation");
     TG_CUDA(d->slots[kBoxes].reserve(size_t(n) * sizeof(int4)), "allocation");
     TG_CUDA(d->slots[kCulls].reserve(size_t(n) * sizeof(float)), "allocation");
     TG_CUDA(d->slots[kScan].reserve(scan_scratch_words(nbins) * sizeof(uint32_t)), "allocation");
@@ -565,6 +566,7 @@ int crater_prepare(tg_device* d, const CraterShapeKernel& k, const CraterRecord*
     bins.total = bins.counts + nbins + 1;
     bins.extrasCount = bins.total + 4;
     bins.extrasList = slot_ptr<uint32_t>(d, kExtrasList);
+    bins.wide = slot_ptr<uint32_t>(d, kWideCraters);
     bins.boxes = slot_ptr<int4>(d, kBoxes);
     bins.culls = slot_ptr<float>(d, kCulls);
     TG_CUDA(cudaMemsetAsync(bins.cursor, 0, words * sizeof(uint32_t), s), "memset");

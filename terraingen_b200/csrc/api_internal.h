@@ -89,6 +89,7 @@ enum Slot {
     kBoulderCursor,
     kBoulderStatus,
     kExtrasList,
+    kWideCraters,
     kRecordCraters,  // the device record builder's plan: craters, then extras
     kRecordCounts,   // its records and floats per crater, then their scans
     kRecordSort,     // the apply order's keys, orders and sort scratch

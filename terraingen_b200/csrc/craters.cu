@@ -35,13 +35,29 @@ constexpr uint32_t kChunk = 96;        // entries per staged chunk (15 KB)
 using namespace binning;
 
 // Binning takes a thread per crater: one of few bins goes through them itself, a block's wider
-// craters are then taken by its warps, and the widest (a 500 m one covers thousands of bins) by the
-// whole block. Numbering the (crater, bin) pairs by a scan and searching it per pair spread them
-// evenly too, at the price of the scan's three launches, a dozen dependent reads a pair and a pass
-// over the craters apart from the lean records' (kernels of 3168 craters on 513^2 cells: 45 us, and
-// of 200,000 on 4097^2: 112 us; 28 and 92 now).
+// craters are then taken by its warps, and the widest (a 500 m one covers thousands of bins) are
+// listed by the count pass and taken a slice of bins to a block, by the whole device. The layers'
+// order puts the widest side by side, so the blocks take craters in turn, and few craters are
+// spread over as many blocks: 128 craters in a row that each cover the 4096 bins of a 2048^2
+// grid took a call of 3.8 ms when one block binned them, and take one of 0.16; 141 craters of
+// 300-500 m on it took 2.6 ms, and take 1.7. Numbering the (crater, bin) pairs by a scan and
+// searching it per pair spread them evenly too (0.27 and 1.7 ms), at the price of the scan's three
+// launches, a dozen dependent reads a pair and a pass over the craters apart from the lean records'
+// (kernels of 3168 craters on 513^2 cells: 45 us, and of 200,000 on 4097^2: 112 us; 23 and 91 now).
 constexpr uint32_t kBinThreads = 128;
 constexpr uint32_t kOwnBins = 4, kWarpBins = 512;
+constexpr uint32_t kBinBlocks = 4 * kSms;   // at least, as far as there are craters
+constexpr uint32_t kWideBlocks = 8 * kSms;  // that share the widest craters
+constexpr uint32_t kWideSlices = 32;        // of them, those that share one crater's bins
+
+// The calling thread's crater of n: the blocks take groups of craters in turn, of a warp's (their
+// records are read side by side) where there are enough for every block.
+__device__ __forceinline__ uint32_t crater_of_thread(uint32_t n) {
+    const uint32_t each = n / kBinBlocks;
+    const uint32_t shift = each > 0u ? min(31u - uint32_t(__clz(int(each))), 5u) : 0u;
+    return (((threadIdx.x >> shift) * gridDim.x + blockIdx.x) << shift) +
+           (threadIdx.x & ((1u << shift) - 1u));
+}
 
 // The bins of a reference-tile box.
 struct BinBox {
@@ -85,7 +101,7 @@ __device__ __forceinline__ void take_bins(uint32_t crater, const BinBox& box, ui
 }
 
 // take_bins for every bin of each of the block's craters (the calling thread's is `mine`, of the
-// bins `box`); every thread of the block calls it.
+// bins `box`) but those of more than kWarpBins; every thread of the block calls it.
 template <typename Reserve, typename Put>
 __device__ __forceinline__ void for_crater_bins(uint32_t mine, const BinBox& box, Reserve reserve,
                                                 Put put) {
@@ -96,34 +112,41 @@ __device__ __forceinline__ void for_crater_bins(uint32_t mine, const BinBox& box
         wideCount = 0;
     }
     __syncthreads();
-    if (box.count > kOwnBins) {
+    if (box.count <= kOwnBins) {
+        take_bins(mine, box, 0u, 1u, reserve, put);
+    } else if (box.count <= kWarpBins) {
         const uint32_t at = atomicAdd(&wideCount, 1u);
         wideCraters[at] = mine;
         wideBoxes[at] = box;
-    } else {
-        take_bins(mine, box, 0u, 1u, reserve, put);
     }
     __syncthreads();
     for (uint32_t c = threadIdx.x / 32u; c < wideCount; c += kBinThreads / 32u) {
-        if (wideBoxes[c].count <= kWarpBins) {
-            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x % 32u, 32u, reserve, put);
-        }
+        take_bins(wideCraters[c], wideBoxes[c], threadIdx.x % 32u, 32u, reserve, put);
     }
-    for (uint32_t c = 0; c < wideCount; ++c) {
-        if (wideBoxes[c].count > kWarpBins) {
-            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x, kBinThreads, reserve, put);
-        }
+}
+
+// take_bins for the listed craters, block `block` of `blocks` (a multiple of kWideSlices).
+template <typename Reserve, typename Put>
+__device__ __forceinline__ void for_wide_bins(const CraterBins& bins, uint32_t block,
+                                              uint32_t blocks, Reserve reserve, Put put) {
+    const uint32_t listed = *bins.total;
+    for (uint32_t c = block / kWideSlices; c < listed; c += blocks / kWideSlices) {
+        const uint32_t crater = bins.wide[c];
+        take_bins(crater, bin_box(bins.boxes[crater]),
+                  block % kWideSlices * kBinThreads + threadIdx.x, kWideSlices * kBinThreads,
+                  reserve, put);
     }
 }
 
 // Per crater: its footprint (the 16-cell tile window and cull radius, as CraterReach and
-// TileLists give it), its LeanCrater with `leans`, and one more entry in each bin it covers.
+// TileLists give it), its LeanCrater with `leans`, and one more entry in each bin it covers or,
+// where those are more than kWarpBins, its place in bins.wide.
 __global__ void __launch_bounds__(kBinThreads)
     crater_footprint_kernel(const CraterShapeKernel k, const CraterRecord* __restrict__ records,
                             uint32_t n, const float* __restrict__ data,
                             const double* __restrict__ footprints, const Grid grid,
                             CraterBins bins, crater::LeanCrater* __restrict__ leans) {
-    const uint32_t i = blockIdx.x * kBinThreads + threadIdx.x;
+    const uint32_t i = crater_of_thread(n);
     BinBox box{0, 0, 0, 0};
     if (i < n) {
         const CraterRecord& r = records[i];
@@ -143,10 +166,24 @@ __global__ void __launch_bounds__(kBinThreads)
             if (leans != nullptr) {
                 leans[i] = crater::lean_crater(k, r, data, i, f.tiles, f.cull);
             }
+            if (box.count > kWarpBins) {
+                bins.wide[atomicAdd(bins.total, 1u)] = i;
+            }
         }
     }
     for_crater_bins(
         i, box,
+        [&](uint32_t bx, uint32_t by) {
+            atomicAdd(bins.counts + by * bins.binsX + bx, 1u);
+            return 0u;
+        },
+        [](uint32_t, uint32_t, uint32_t, uint32_t) {});
+}
+
+// The count pass's listed craters.
+__global__ void __launch_bounds__(kBinThreads) crater_wide_count_kernel(CraterBins bins) {
+    for_wide_bins(
+        bins, blockIdx.x, gridDim.x,
         [&](uint32_t bx, uint32_t by) {
             atomicAdd(bins.counts + by * bins.binsX + bx, 1u);
             return 0u;
@@ -184,7 +221,7 @@ __global__ void __launch_bounds__(kBinThreads)
     if (!crater_bins_usable(bins)) {
         return;
     }
-    const uint32_t mine = blockIdx.x * kBinThreads + threadIdx.x;
+    const uint32_t mine = crater_of_thread(n);
     BinBox box{0, 0, 0, 0};
     if (mine < n) {
         box = bin_box(bins.boxes[mine]);
@@ -193,8 +230,7 @@ __global__ void __launch_bounds__(kBinThreads)
         const uint32_t b = by * bins.binsX + bx;
         return bins.counts[b] + atomicAdd(bins.cursor + b, 1u);
     };
-    for_crater_bins(mine, box, reserve, [&](uint32_t crater, uint32_t slot, uint32_t bx,
-                                            uint32_t by) {
+    const auto put = [&](uint32_t crater, uint32_t slot, uint32_t bx, uint32_t by) {
         if (slot >= bins.capacity) {
             return;  // the total fits the capacity (checked above); never taken
         }
@@ -223,7 +259,12 @@ __global__ void __launch_bounds__(kBinThreads)
         dst[9] = make_int4(int(uint32_t(t.x) | (uint32_t(t.y) << 16)),
                            int(uint32_t(t.z) | (uint32_t(t.w) << 16)),
                            __float_as_int(bins.culls[crater]), int(crater));
-    });
+    };
+    for_crater_bins(mine, box, reserve, put);
+    const uint32_t sharing = gridDim.x / kWideSlices * kWideSlices;
+    if (blockIdx.x < sharing) {
+        for_wide_bins(bins, blockIdx.x, sharing, reserve, put);
+    }
 }
 
 // (amplitude, phase) of each record's outline harmonics as (amplitude cos phase,
@@ -1074,6 +1115,22 @@ cudaError_t launch_exclusive_scan(uint32_t* counts, uint32_t n, uint32_t* scratc
     return cudaGetLastError();
 }
 
+namespace {
+
+// Whether a crater may cover more than kWarpBins bins: only on a grid that has them.
+bool may_list(const CraterBins& bins) {
+    return bins.binsX * bins.binsY > kWarpBins;
+}
+
+// The blocks of a binning pass over n craters; where craters may be listed, all that share them.
+uint32_t bin_blocks(uint32_t n, const CraterBins& bins) {
+    static_assert(kWideBlocks % kWideSlices == 0, "whole groups of blocks share a crater");
+    const uint32_t spread = may_list(bins) ? kWideBlocks : std::min(n, kBinBlocks);
+    return std::max((n + kBinThreads - 1) / kBinThreads, spread);
+}
+
+}  // namespace
+
 cudaError_t launch_crater_count(const CraterShapeKernel& k, const CraterRecord* records,
                                 uint32_t n, const float* data, const double* footprints,
                                 const Grid& grid, const CraterBins& bins, void* leans,
@@ -1082,8 +1139,13 @@ cudaError_t launch_crater_count(const CraterShapeKernel& k, const CraterRecord* 
     if (n == 0) {
         return cudaSuccess;
     }
-    crater_footprint_kernel<<<(n + kBinThreads - 1) / kBinThreads, kBinThreads, 0, stream>>>(
+    crater_footprint_kernel<<<bin_blocks(n, bins), kBinThreads, 0, stream>>>(
         k, records, n, data, footprints, grid, bins, static_cast<crater::LeanCrater*>(leans));
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess || !may_list(bins)) {
+        return err;
+    }
+    crater_wide_count_kernel<<<kWideBlocks, kBinThreads, 0, stream>>>(bins);
     return cudaGetLastError();
 }
 
@@ -1093,7 +1155,7 @@ cudaError_t launch_crater_scatter(const CraterShapeKernel& k, const CraterRecord
     if (n == 0) {
         return cudaSuccess;
     }
-    crater_bin_scatter_kernel<<<(n + kBinThreads - 1) / kBinThreads, kBinThreads, 0, stream>>>(
+    crater_bin_scatter_kernel<<<bin_blocks(n, bins), kBinThreads, 0, stream>>>(
         k, records, n, static_cast<const crater::LeanCrater*>(leans), grid, bins);
     return cudaGetLastError();
 }

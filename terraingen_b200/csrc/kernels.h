@@ -10,6 +10,8 @@
 
 namespace tgb {
 
+constexpr uint32_t kSms = 148;  // of a B200
+
 // A non-rotated grid's GeoTransform (include/terraingen/raster/geo_transform.h:17-35): cell
 // (col, row) has its center at originX + (col + 0.5) * pixelWidth + (row + 0.5) * rowRotation,
 // originY + (col + 0.5) * colRotation + (row + 0.5) * pixelHeight.
@@ -76,7 +78,9 @@ struct CraterBins {
     uint32_t* cursor;    // [bins]
     BinEntry* entries;   // [capacity]
     uint32_t capacity;
-    uint32_t* total;     // [4], zeroed: unused, flags, the pairs evaluated (64 bits, aligned)
+    uint32_t* total;     // [4], zeroed: the craters listed in `wide`, flags, the pairs evaluated
+                         // (64 bits, aligned)
+    uint32_t* wide;      // [craters]: those that cover the most bins, binned by the whole device
     int4* boxes;         // [craters] reference-tile box per crater (x0, x1, y0, y1); empty: x0 > x1
     float* culls;        // [craters] cull distance per crater
     uint32_t firstBin;   // the bin of a launch's first block (a strip of bin rows)
