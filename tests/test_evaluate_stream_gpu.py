@@ -1,5 +1,6 @@
 """tg_evaluate on device memory bins its layers on a stream of the device's own, beside the source on
-the caller's: binning that has to grow its entries and run again."""
+the caller's: binning that has to grow its entries and run again, and inputs that the caller's
+stream is still to write."""
 
 import numpy as np
 import pytest
@@ -60,3 +61,30 @@ def test_growing_on_device_memory_gives_the_same_heights():
         fresh.evaluate(grid, host, fractals=scene[3], craters=scene[1], boulders=scene[2],
                        boulder_width=grid.pixel)
     np.testing.assert_array_equal(first.cpu().numpy(), host)
+
+
+def test_inputs_the_stream_is_still_to_write_are_waited_for(device):
+    import torch
+
+    scene = _scene()
+    grid, _, _, _ = scene
+    ready = _tensors(*scene[1:3])
+    want = _evaluate(device, scene, ready, torch.empty((grid.height, grid.width), device="cuda"))
+    # Other inputs of the same sizes, as valid: the craters and boulders without any relief.
+    flat = _tensors(*scene[1:3])
+    records, _, _, stones = flat
+    records.view(-1, 144)[:] = records.view(-1, 144)[0].clone()
+    flat[2].view(-1, 3)[:] = torch.tensor([1e6, 1e6, 1.0], dtype=torch.float64, device="cuda")
+    stones[:, 0] = 1e6
+    other = _evaluate(device, scene, flat, torch.empty_like(want))
+    assert not torch.equal(other, want)
+    got = torch.empty_like(want)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)  # 10 ms at 2 GHz, before the copies
+        for to, of in zip(flat, ready):
+            to.copy_(of)
+        _evaluate(device, scene, flat, got)
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
