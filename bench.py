@@ -218,8 +218,34 @@ def cpu_sample(steps, warmup, window, quiet=False):
     return grid.cells / per / 1e6, per, len(times), grid
 
 
+def reference_missing():
+    """Why the reference's CPU path cannot be timed here, or None: its library is built from the
+    reference's own sources, which not every checkout has."""
+    from oracle import harness as H
+
+    name = "libtgref.so"
+    return None if H.available(name) else (f"oracle/_ref/{name} is not built (it needs the "
+                                           "reference's sources)")
+
+
+def cpu_baseline(window):
+    """The line's cpu_baseline: one evaluation of the reference's CPU path, or why there is none."""
+    missing = reference_missing()
+    if missing:
+        return {"value": None, "unit": UNIT, "cores": os.cpu_count(), "kind": "reference",
+                "unavailable": missing}
+    value, per, _, grid = cpu_sample(1, 1, window)
+    return {"value": round(value, 3), "unit": UNIT, "cores": os.cpu_count(), "kind": "reference",
+            "sample": f"{grid.width}x{grid.height} window of the same terrain on the reference "
+                      f"CPU path, {per * 1e3:.0f} ms"}
+
+
 def run_reference(args, rank, world):
     if rank != 0:
+        return
+    missing = reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return
     value, per, n, grid = cpu_sample(args.steps, args.warmup, args.cpu_window)
     cores = os.cpu_count()
@@ -1042,7 +1068,7 @@ def main():
     # extras pass; boulders: count, bin scan, scatter, bake.
     launches = (1 + (6 + scan_launches(len(w.crater_records)) + scan_launches(nbins)) +
                 (3 + scan_launches(nbins)))
-    cpu_value, cpu_per, cpu_n, cpu_grid = cpu_sample(1, 1, args.cpu_window)
+    cpu = cpu_baseline(args.cpu_window)
     dropin = dropin_leg(args.cpu_window)
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": UNIT, "n_gpus": world,
@@ -1080,10 +1106,7 @@ def main():
                      "others": {k: {"ms": round(v[1], 4),
                                     "achieved": round(v[0] / (v[1] * 1e-3) / 1e12, 3)}
                                 for k, v in work.items() if k != dominant}},
-        "cpu_baseline": {"value": round(cpu_value, 3), "unit": UNIT, "cores": os.cpu_count(),
-                         "kind": "reference",
-                         "sample": f"{cpu_grid.width}x{cpu_grid.height} window of the same terrain "
-                                   f"on the reference CPU path, {cpu_per * 1e3:.0f} ms"},
+        "cpu_baseline": cpu,
         "fp64": fp64,
         "e2e": {**e2e, "matches_device_path": same},
         "dropin": dropin,
