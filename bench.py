@@ -273,6 +273,13 @@ def scan_launches(n):
     return 1 if blocks == 1 else 2 + scan_launches(blocks)
 
 
+def step_launches(nbins):
+    """Kernel launches of one step on a grid of `nbins` bins: the source; the craters' footprints,
+    the count of the widest (on grids of more than 512 bins), the bins' scan, scatter, lean shaping
+    and extras pass; the boulders' count, scan, scatter and bake."""
+    return (1 + (4 + (nbins > 512) + scan_launches(nbins)) + (3 + scan_launches(nbins)))
+
+
 def batched_form(dev, args, rank, world, alu_peak):
     """The batched form on uneven tiles (tiles4096): every rank its own 4096 tiles, evaluated in
     one persistent launch replayed from CUDA graphs, against the plain per-tile path on the same
@@ -1064,10 +1071,6 @@ def main():
     achieved = ops / (ms * 1e-3) / 1e12
     peak = alu_peak / 1e12
     nbins = ((w.grid.width + 31) // 32) * ((w.grid.height + 31) // 32)
-    # noise; craters: footprints, pair scan, count, bin scan, lean records, scatter, lean shape,
-    # extras pass; boulders: count, bin scan, scatter, bake.
-    launches = (1 + (6 + scan_launches(len(w.crater_records)) + scan_launches(nbins)) +
-                (3 + scan_launches(nbins)))
     cpu = cpu_baseline(args.cpu_window)
     dropin = dropin_leg(args.cpu_window)
     line = {
@@ -1110,7 +1113,7 @@ def main():
         "fp64": fp64,
         "e2e": {**e2e, "matches_device_path": same},
         "dropin": dropin,
-        "gpu_launches": int(launches * args.steps),
+        "gpu_launches": int(step_launches(nbins) * args.steps),
         "clocks": clocks.summary(),
         "forms": forms,
     }

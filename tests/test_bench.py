@@ -27,3 +27,13 @@ def test_the_line_keeps_its_measurements_without_the_reference(no_reference):
     baseline = bench.cpu_baseline(65)
     assert baseline["value"] is None and "libtgref.so" in baseline["unavailable"]
     assert "unavailable" in bench.dropin_leg(65)
+
+
+@pytest.mark.parametrize("side, kernels", [
+    (513, ["fbm", "crater_footprint", "scan_block", "crater_bin_scatter", "crater_lean_shape",
+           "crater_extras", "boulder_count", "scan_block", "boulder_scatter", "boulder_bake"]),
+    (4097, ["fbm", "crater_footprint", "crater_wide_count", "scan_block", "scan_block", "scan_add",
+            "crater_bin_scatter", "crater_lean_shape", "crater_extras", "boulder_count",
+            "scan_block", "scan_block", "scan_add", "boulder_scatter", "boulder_bake"])])
+def test_a_steps_launches_are_the_profilers_list(side, kernels):
+    assert bench.step_launches(((side + 31) // 32) ** 2) == len(kernels)
