@@ -40,10 +40,10 @@ METRIC = "Mcells/s at <=1e-3 m err: served/batched vs plain GPU; p50/p99 tile ms
 UNIT = "Mcells/s"
 SIDE = 4097
 PIXEL = 0.5
-# Counted from terraingen_b200/csrc/noise_math.cuh (perlin_fbm2), per cell and octave: octave
-# key hash and offsets 21, turn 6, lattice 4, split 6, 4 corner hashes 45, 4 gradients 56 plus 2
-# offsets, 2 fades 14, lerps and scale 10, sums 5, turn update 6, loop 3.
-NOISE_OPS_PER_CELL_OCTAVE = 180
+# Counted from terraingen_b200/csrc/noise.cu (fbm_kernel), per cell and octave whose corners'
+# gradients are at hand: turn 6, lattice position 4, split 6, offsets 2, 4 gradients x 3, 2 fades x
+# 7, 3 lerps x 3, scale 1, sum 2: 56, and a look at each corner's gradient.
+NOISE_OPS_PER_CELL_OCTAVE = 60
 # Counted from the reference's crater kernel (include/terraingen/layers/kernels/craters.h:
 # KernelProfileDistance, ComplexProfileHeight / FassettThomsonShape, ApplyCraterKernel) per
 # (cell, crater) pair of the synthetic terrain's craters (11 outline harmonics; a transcendental
@@ -52,9 +52,9 @@ NOISE_OPS_PER_CELL_OCTAVE = 180
 # 8, resolution and the add 2: 104, plus the ellipse of 5 % of craters (10): 105.
 CRATER_OPS_PER_PAIR = 105
 # Thread instructions the lean crater kernel executes per pair, measured with ncu on a tile of
-# this workload's make (smsp__inst_executed x active lanes / pairs: 580.1 M x 28.37 / 58,126,370):
+# this workload's make (smsp__inst_executed x active lanes / pairs: 607.2 M x 28.20 / 58,126,370):
 # the issue-rate view of the same work (loads, the boxes' cells, compares and selects).
-CRATER_THREAD_INST_PER_PAIR = 283
+CRATER_THREAD_INST_PER_PAIR = 295
 # Counted from terraingen_b200/csrc/boulders.cu per (cell, boulder) pair: window test 6, offset
 # and hypot 12, dome band average (2 sqrt, 2 asin, clamps) 60, max-composite 4; FP64.
 BOULDER_OPS_PER_PAIR = 82

@@ -37,3 +37,10 @@ def test_the_line_keeps_its_measurements_without_the_reference(no_reference):
             "scan_block", "scan_block", "scan_add", "boulder_scatter", "boulder_bake"])])
 def test_a_steps_launches_are_the_profilers_list(side, kernels):
     assert bench.step_launches(((side + 31) // 32) ** 2) == len(kernels)
+
+
+def test_operations_are_those_of_the_cases():
+    from perf import cases
+
+    assert bench.NOISE_OPS_PER_CELL_OCTAVE == cases._OCTAVE
+    assert bench.CRATER_OPS_PER_PAIR == cases._CRATER
