@@ -705,8 +705,9 @@ __device__ __forceinline__ float4 gradient3_of(uint32_t h) {
     return g;
 }
 
-// PerlinNoise3 at a cell (perlin.h:113-128) with its corners' directions read from a shared table:
-// selecting them per corner kept the integer pipe 77 % busy.
+// PerlinNoise3 at a cell (perlin.h:113-128; corner keys x, y, z + pcg(seed), the last term `key`)
+// with its corners' directions read from a shared table: selecting them per corner kept the integer
+// pipe 77 % busy.
 __device__ __forceinline__ float perlin3_table(const noise::Cell3& c, uint32_t key,
                                                const float4* directions) {
     uint32_t ax[2], ay[2], az[2];

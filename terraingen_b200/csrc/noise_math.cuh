@@ -459,23 +459,6 @@ __device__ __forceinline__ Cell3 split3_precise(double x, double y, double z) {
                  float(x - cx), float(y - cy), float(z - cz)};
 }
 
-// PerlinNoise3 at a cell (perlin.h:113-128): corner keys (x, y, z + pcg(seed)).
-__device__ __forceinline__ float perlin3_cell(const Cell3& c, uint32_t seed) {
-    const uint32_t key = pcg(seed);
-    const uint32_t ix = uint32_t(c.ix), iy = uint32_t(c.iy), iz = uint32_t(c.iz);
-    float k[8];
-#pragma unroll
-    for (uint32_t corner = 0; corner < 8u; ++corner) {
-        const uint32_t dx = corner & 1u, dy = (corner >> 1u) & 1u, dz = corner >> 2u;
-        const uint32_t h = pcg3d(U3{ix + dx, iy + dy, iz + dz + key}).x;
-        k[corner] = gradient3(h, c.fx - float(dx), c.fy - float(dy), c.fz - float(dz));
-    }
-    const float u = fade(c.fx), v = fade(c.fy), w = fade(c.fz);
-    const float near = lerp(v, lerp(u, k[0], k[1]), lerp(u, k[2], k[3]));
-    const float far = lerp(v, lerp(u, k[4], k[5]), lerp(u, k[6], k[7]));
-    return sclamp(lerp(w, near, far), -1.0f, 1.0f);
-}
-
 // One corner of a 3D simplex (SimplexCorner3, simplex.h:27).
 __device__ __forceinline__ float simplex_corner3(uint32_t ci, uint32_t cj, uint32_t ck, float dx,
                                                  float dy, float dz, uint32_t key) {
@@ -595,7 +578,8 @@ __device__ __forceinline__ WorleyD worley3_cell(const Cell3& c, uint32_t seed) {
     return WorleyD{sqrtf(d1), sqrtf(d2), 2.0f * unit(nearest) - 1.0f};
 }
 
-// One octave of any 3D basis (BasisNoise3, fractal.h:115).
+// One octave of a 3D basis other than Perlin's, which reads its directions from a table the kernel
+// holds (BasisNoise3, fractal.h:115).
 __device__ __forceinline__ float basis3(uint32_t basis, const Cell3& c, uint32_t seed) {
     const float kInvSqrt3 = 0.577350269189625765f;
     const float kInvSqrt6 = 0.408248290463863016f;
@@ -612,10 +596,8 @@ __device__ __forceinline__ float basis3(uint32_t basis, const Cell3& c, uint32_t
         const WorleyD d = worley3_cell(c, seed);
         return 2.0f * smin((d.f2 - d.f1) * kInvSqrt6, 1.0f) - 1.0f;
     }
-    case kBasisVoronoi:
+    default:  // kBasisVoronoi
         return worley3_cell(c, seed).value;
-    default:
-        return perlin3_cell(c, seed);
     }
 }
 
