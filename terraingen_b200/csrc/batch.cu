@@ -1335,7 +1335,7 @@ int occupancy() {
 
 uint32_t grid_for(uint32_t items, uint32_t perBlock) {
     const uint64_t blocks = (uint64_t(items) + perBlock - 1) / perBlock;
-    return uint32_t(blocks < 1 ? 1 : (blocks > 148u * 32u ? 148u * 32u : blocks));
+    return uint32_t(blocks < 1 ? 1 : (blocks > 32u * kSms ? 32u * kSms : blocks));
 }
 
 }  // namespace

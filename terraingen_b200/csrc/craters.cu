@@ -1207,7 +1207,7 @@ cudaError_t launch_crater_shape(const CraterShapeKernel& k, const CraterRecord* 
             if (err != cudaSuccess) {
                 return err;
             }
-            const uint32_t grid2 = std::min(nbins, 148u * 4u);
+            const uint32_t grid2 = std::min(nbins, 4u * kSms);
             crater_extras_kernel<<<grid2, kShapeThreads, 0, stream>>>(
                 k, records, data, lean, grid, nodata, strip, nbins, heights);
         }

@@ -936,13 +936,15 @@ cudaError_t launch_noise(const FractalStack& stack, const Grid& grid, const Posi
         }
         oct.total = total;
         oct.one = 1.0f;
-        // Rows a thread takes: 8 amortize a block's tables best (2049^2 cells: 81 us against 106
-        // with 2), as long as that leaves the SMs several blocks each; a small grid's octaves
-        // run in parallel over its cells instead of in series over a few blocks (257^2: the
-        // kernel took 17 us with 8 rows a thread; with 2 the whole call takes 12).
+        // Rows a thread takes: 8 amortize a block's tables best (2049^2 cells: 83 us against 102
+        // with 2), from two and a half blocks of 8 rows an SM on. Below, a grid's octaves run in
+        // parallel over its cells instead of in series over a few blocks (257^2: the kernel took
+        // 17 us with 8 rows; with 2 the whole call takes 12). Us a call with 8 and with 2 on either
+        // side of the line: 769^2 21.6 and 19.8, 833^2 21.6 and 21.8, 865^2 21.6 and 23.8, 1025^2
+        // 25.9 and 30.1, 1537^2 48.4 and 60.7.
         const size_t columns = (grid.width + kBlockX - 1) / kBlockX;
         const size_t lines = (grid.height + kBlockY - 1) / kBlockY;
-        if (columns * lines >= 8 * 1184) {
+        if (columns * lines >= 5 * 8 * size_t(kSms) / 2) {
             launch_fbm<8>(oct, grid, at, fill, elevation, nodata, heights, stream);
         } else {
             launch_fbm<2>(oct, grid, at, fill, elevation, nodata, heights, stream);

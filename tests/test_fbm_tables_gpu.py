@@ -70,3 +70,21 @@ def test_origins_that_are_no_floats_give_nan(device, origin):
                                        *origin, out.ctypes.data, N.NoData(0, 0.0),
                                        N.TG_MEMORY_HOST, None))
     assert np.isnan(out).all()
+
+
+@pytest.mark.parametrize("side", [833, 865])
+def test_a_grid_is_its_windows_on_both_sides_of_the_rows_rule(device, side):
+    """Two rows a thread on the window, and on the smaller grid; eight on the larger."""
+    f = np.array([fractal(seed=9, wavelength=300.0, amplitude=7.0, octaves=9)])
+
+    def source(x0, y0, n):
+        out = np.zeros((n, n), np.float32)
+        N.check(device._lib.tg_noise_source(device._handle, f.ctypes.data, 1, 0.0,
+                                            C.byref(N.Grid(n, n, x0, 0.5, 0.0, y0, 0.0, -0.5)),
+                                            out.ctypes.data, N.TG_MEMORY_HOST, None))
+        return out
+
+    whole = source(-100.0, 50.0, side)
+    for row, col in ((0, 0), (333, 417), (side - 61, side - 61)):
+        np.testing.assert_array_equal(source(-100.0 + 0.5 * col, 50.0 - 0.5 * row, 61),
+                                      whole[row:row + 61, col:col + 61])
