@@ -275,9 +275,9 @@ def scan_launches(n):
 
 def step_launches(nbins):
     """Kernel launches of one step on a grid of `nbins` bins: the source; the craters' footprints,
-    the count of the widest (on grids of more than 512 bins), the bins' scan, scatter, lean shaping
+    the count of the widest (on grids of more than 8192 bins), the bins' scan, scatter, lean shaping
     and extras pass; the boulders' count, scan, scatter and bake."""
-    return (1 + (4 + (nbins > 512) + scan_launches(nbins)) + (3 + scan_launches(nbins)))
+    return (1 + (4 + (nbins > 8192) + scan_launches(nbins)) + (3 + scan_launches(nbins)))
 
 
 def batched_form(dev, args, rank, world, alu_peak):
@@ -507,7 +507,7 @@ def dem_form(dev, args, rank, world):
                     "+-2000 m) refined 10x by "
                     "diamond-square (F 2.2, scale 1.5 m, 4 levels, bilinear) to 20481^2 at 0.5 m "
                     "as 2x2 patches (own seeds, 64-cell overlap) chained with Height seams "
-                    "(3 L = 64 cells, 4-level V-cycle, Jacobi smoother, FP64 PCG to 1e-10), then "
+                    "(3 L = 64 cells, 4-level V-cycle, Chebyshev smoother, FP64 PCG to 1e-10), then "
                     "2,000,000 craters (D^-2 on [1, 100] m)",
         "cells_per_gpu": w.cells, "craters": int(len(w.crater_records)),
         "value": round(value, 3), "unit": UNIT,

@@ -17,10 +17,9 @@
 // window touches (apply.cpp:119-143, 199-222), whatever the bin size here.
 //
 // Accumulation: without a datum a crater adds resolution * shaped relief independently of the
-// height beneath it (apply_test.cpp:276-286), so the contributions are summed in an FP64
-// accumulator. Each contribution is an FP32 value and the sum stays far inside 53 bits, so the
-// accumulation is error-free: the result is the FP32 rounding of the exact sum, independent of
-// the order atomics put the entries in, so every run gives the same bits.
+// height beneath it (apply_test.cpp:276-286), so the contributions, FP32 values each rounded once
+// to 64-bit fixed point, are summed as integers: exactly, independent of the order atomics put the
+// entries in, so every run gives the same bits.
 #include "binning.cuh"
 #include "crater_math.cuh"
 #include "kernels.h"
@@ -35,17 +34,17 @@ constexpr uint32_t kChunk = 96;        // entries per staged chunk (15 KB)
 using namespace binning;
 
 // Binning takes a thread per crater: one of few bins goes through them itself, a block's wider
-// craters are then taken by its warps, and the widest (a 500 m one covers thousands of bins) are
-// listed by the count pass and taken a slice of bins to a block, by the whole device. The layers'
-// order puts the widest side by side, so the blocks take craters in turn, and few craters are
-// spread over as many blocks: 128 craters in a row that each cover the 4096 bins of a 2048^2
+// craters are then taken by its warps, the still wider (a 500 m one covers thousands of bins) by
+// the block, and those of more than 8192 bins are listed by the count pass and taken a slice of
+// bins to a block, by the whole device. The layers' order puts the widest side by side, so the
+// blocks take craters in turn, and few craters are spread over as many blocks: 128 craters in a row that each cover the 4096 bins of a 2048^2
 // grid took a call of 3.8 ms when one block binned them, and take one of 0.16; 141 craters of
 // 300-500 m on it took 2.6 ms, and take 1.7. Numbering the (crater, bin) pairs by a scan and
 // searching it per pair spread them evenly too (0.27 and 1.7 ms), at the price of the scan's three
 // launches, a dozen dependent reads a pair and a pass over the craters apart from the lean records'
 // (kernels of 3168 craters on 513^2 cells: 45 us, and of 200,000 on 4097^2: 112 us; 23 and 91 now).
 constexpr uint32_t kBinThreads = 128;
-constexpr uint32_t kOwnBins = 4, kWarpBins = 512;
+constexpr uint32_t kOwnBins = 4, kWarpBins = 512, kBlockBins = 8192;
 constexpr uint32_t kBinBlocks = 4 * kSms;   // at least, as far as there are craters
 constexpr uint32_t kWideBlocks = 8 * kSms;  // that share the widest craters
 constexpr uint32_t kWideSlices = 32;        // of them, those that share one crater's bins
@@ -101,7 +100,7 @@ __device__ __forceinline__ void take_bins(uint32_t crater, const BinBox& box, ui
 }
 
 // take_bins for every bin of each of the block's craters (the calling thread's is `mine`, of the
-// bins `box`) but those of more than kWarpBins; every thread of the block calls it.
+// bins `box`) but those of more than kBlockBins; every thread of the block calls it.
 template <typename Reserve, typename Put>
 __device__ __forceinline__ void for_crater_bins(uint32_t mine, const BinBox& box, Reserve reserve,
                                                 Put put) {
@@ -114,14 +113,21 @@ __device__ __forceinline__ void for_crater_bins(uint32_t mine, const BinBox& box
     __syncthreads();
     if (box.count <= kOwnBins) {
         take_bins(mine, box, 0u, 1u, reserve, put);
-    } else if (box.count <= kWarpBins) {
+    } else if (box.count <= kBlockBins) {
         const uint32_t at = atomicAdd(&wideCount, 1u);
         wideCraters[at] = mine;
         wideBoxes[at] = box;
     }
     __syncthreads();
     for (uint32_t c = threadIdx.x / 32u; c < wideCount; c += kBinThreads / 32u) {
-        take_bins(wideCraters[c], wideBoxes[c], threadIdx.x % 32u, 32u, reserve, put);
+        if (wideBoxes[c].count <= kWarpBins) {
+            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x % 32u, 32u, reserve, put);
+        }
+    }
+    for (uint32_t c = 0; c < wideCount; ++c) {
+        if (wideBoxes[c].count > kWarpBins) {
+            take_bins(wideCraters[c], wideBoxes[c], threadIdx.x, kBinThreads, reserve, put);
+        }
     }
 }
 
@@ -140,7 +146,7 @@ __device__ __forceinline__ void for_wide_bins(const CraterBins& bins, uint32_t b
 
 // Per crater: its footprint (the 16-cell tile window and cull radius, as CraterReach and
 // TileLists give it), its LeanCrater with `leans`, and one more entry in each bin it covers or,
-// where those are more than kWarpBins, its place in bins.wide.
+// where those are more than kBlockBins, its place in bins.wide.
 __global__ void __launch_bounds__(kBinThreads)
     crater_footprint_kernel(const CraterShapeKernel k, const CraterRecord* __restrict__ records,
                             uint32_t n, const float* __restrict__ data,
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(kBinThreads)
             if (leans != nullptr) {
                 leans[i] = crater::lean_crater(k, r, data, i, f.tiles, f.cull);
             }
-            if (box.count > kWarpBins) {
+            if (box.count > kBlockBins) {
                 bins.wide[atomicAdd(bins.total, 1u)] = i;
             }
         }
@@ -719,7 +725,7 @@ __device__ __forceinline__ LeanBox lean_box(const crater::LeanCrater& l, float x
 // [1, 500] m: 442 us; 358 a pair with complex craters, 818 us). Here the cells of all staged
 // craters' boxes are numbered in one sequence (a scan of the boxes' sizes) and the block's threads
 // take them in turn: four of five of the sequence's cells are pairs, and 87 % of the lanes that
-// shape one have one. 283 a pair with complex craters, 683 us; 331 us without. It issues on 77 % of
+// shape one have one. 295 a pair with complex craters, 698 us; 325 us without. It issues on 79 % of
 // cycles. Accumulation as above, in the block's accumulators. Four CTAs of 256 threads per SM
 // (64 registers); five with spills are no faster.
 __global__ void __launch_bounds__(kShapeThreads, 4)
@@ -1117,9 +1123,10 @@ cudaError_t launch_exclusive_scan(uint32_t* counts, uint32_t n, uint32_t* scratc
 
 namespace {
 
-// Whether a crater may cover more than kWarpBins bins: only on a grid that has them.
+// Whether a crater may cover more than kBlockBins bins: only on a grid that has them. (Smaller
+// grids do without the listed craters' launch, 3 us; a block takes 8192 bins in 11.)
 bool may_list(const CraterBins& bins) {
-    return bins.binsX * bins.binsY > kWarpBins;
+    return bins.binsX * bins.binsY > kBlockBins;
 }
 
 // The blocks of a binning pass over n craters; where craters may be listed, all that share them.

@@ -43,6 +43,25 @@ def test_a_layer_of_wide_craters_is_its_windows(device, smallest, general):
         np.testing.assert_array_equal(part, whole[row:row + 256, col:col + 256])
 
 
+@pytest.mark.parametrize("general", [False, True], ids=["lean", "general"])
+def test_craters_of_more_bins_than_a_block_takes_are_their_windows(device, general):
+    """A grid of 9216 bins under craters that reach over all of it, among others."""
+    spec = centered(3072, 3072, 0.5)
+    batch = W.crater_batch(W.crater_population(5, 20.0, 100.0, 4000.0), spec)
+    foot = batch[3].reshape(-1, 3)
+    covering = np.abs(foot[:, :2]).max(axis=1) + 768.0 < foot[:, 2]
+    assert 1 <= covering.sum() < len(foot)
+    batch[0]["mantling"] = 1e-30 if general else 0.0
+    grid = spec.native()
+    whole = np.zeros((3072, 3072), np.float32)
+    _apply(device, batch, grid, whole)
+    assert np.abs(whole).max() > 1.0
+    for col, row in ((0, 0), (1504, 2016), (2816, 2816)):
+        part = np.zeros((256, 256), np.float32)
+        _apply(device, batch, _window(grid, col, row, 256), part)
+        np.testing.assert_array_equal(part, whole[row:row + 256, col:col + 256])
+
+
 def _milliseconds(device, batch, spec):
     import torch
 
