@@ -936,15 +936,27 @@ cudaError_t launch_noise(const FractalStack& stack, const Grid& grid, const Posi
         }
         oct.total = total;
         oct.one = 1.0f;
-        // Rows a thread takes: 8 amortize a block's tables best (2049^2 cells: 83 us against 102
-        // with 2), from two and a half blocks of 8 rows an SM on. Below, a grid's octaves run in
-        // parallel over its cells instead of in series over a few blocks (257^2: the kernel took
-        // 17 us with 8 rows; with 2 the whole call takes 12). Us a call with 8 and with 2 on either
-        // side of the line: 769^2 21.6 and 19.8, 833^2 21.6 and 21.8, 865^2 21.6 and 23.8, 1025^2
-        // 25.9 and 30.1, 1537^2 48.4 and 60.7.
+        // Rows a thread takes: 8 amortize a block's tables best, once there are enough blocks; a
+        // small grid's octaves run in parallel over its cells instead of in series over a few
+        // blocks (257^2: the kernel took 17 us with 8 rows; with 2 the whole call takes 12), and
+        // octaves that are hashed per cell gain nothing from more rows. So 8 rows from two and a
+        // half blocks of them an SM on where at least half of the octaves are tabled, else from
+        // eight. Us a call with 8 and with 2: 8 octaves, all tabled, 769^2 21.6 and 19.8, 833^2 21.6
+        // and 21.8, 865^2 21.6 and 23.8, 1537^2 48.4 and 60.7; 24 octaves, most of them hashed,
+        // 1281^2 170 and 163, 1537^2 229 and 227.
         const size_t columns = (grid.width + kBlockX - 1) / kBlockX;
         const size_t lines = (grid.height + kBlockY - 1) / kBlockY;
-        if (columns * lines >= 5 * 8 * size_t(kSms) / 2) {
+        const size_t most = columns * lines / 8;  // blocks of 8 rows a thread
+        bool eight = most >= 8 * size_t(kSms);
+        if (!eight && 2 * most >= 5 * size_t(kSms)) {
+            place_tables(oct, grid, at, kBlockY * 8);
+            int tabled = 0;
+            for (uint32_t bits = oct.tabled; bits != 0u; bits &= bits - 1u) {
+                ++tabled;
+            }
+            eight = 2 * tabled >= oct.count;
+        }
+        if (eight) {
             launch_fbm<8>(oct, grid, at, fill, elevation, nodata, heights, stream);
         } else {
             launch_fbm<2>(oct, grid, at, fill, elevation, nodata, heights, stream);
