@@ -761,8 +761,10 @@ __device__ __forceinline__ noise::Sums body_octaves(const BodyLayout& stack, uin
 // longitude and each row's latitude, then the stack in 3D. The octaves' turns, frequencies and
 // keys are made once on the host, by the recurrences in double that Fractal3 runs per cell. It is
 // bound by issuing instructions (84 % of cycles). 1025^2 cells, 8 octaves: 146 us when each cell
-// multiplied its own matrices, 120 with the host's, 82 with the corners' directions from a table.
-__global__ void __launch_bounds__(128)
+// multiplied its own matrices, 120 with the host's, 82 with the corners' directions from a table
+// (calls of 81.3 us with room for seven blocks an SM, 82.5 without that bound, 83 to 85 with eight
+// to ten).
+__global__ void __launch_bounds__(128, 7)
     noise_body_kernel(const __grid_constant__ BodyLayout stack, float elevation, uint32_t width,
                       uint32_t height, const double* __restrict__ lons,
                       const double* __restrict__ lats, double radius,
