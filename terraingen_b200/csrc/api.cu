@@ -1150,7 +1150,7 @@ int tg_evaluate(tg_device* d, const tg_terrain* t, const tg_grid* grid, float* h
     // Terrain::Fill: the source, then each layer in order (src/pipeline/terrain.cpp:299-331).
     const Positions origin{0.0, 0.0, nullptr, nullptr};
     // The layers' binning needs no heights: it runs on the device's side stream beside the source's
-    // kernels (4097^2 cells, 200,000 craters and 1,000,000 boulders: 130 us of small kernels that
+    // kernels (4097^2 cells, 200,000 craters and 1,000,000 boulders: 135 us of small kernels that
     // leave most SMs idle), behind what the caller's stream holds already.
     const cudaStream_t side = d->copyStream;
     const bool layers = t->n_craters > 0 || t->n_boulders > 0;

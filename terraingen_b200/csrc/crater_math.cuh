@@ -1235,10 +1235,10 @@ __device__ __forceinline__ float lean_height(const CraterShapeKernel& k, const L
 // round dome in place of massifs); `reached` is false beyond its reach.
 //
 // The kernel is bound by issuing instructions, so the distance and the direction come from one
-// reciprocal square root, the profile's quotients are products by reciprocals, most of them made
-// once per crater, and the quotient by the outline's scale is the fast divide: each within a few
-// ulp of the correctly rounded operation, far inside the heights' 1e-3 m tolerance and the cull
-// radius's 1e-5 relative margin.
+// reciprocal square root, the division by the radius is a product by a reciprocal made once per
+// crater and the quotient by the outline's scale is the fast divide: each within a few ulp of the
+// correctly rounded operation, far inside the heights' 1e-3 m tolerance and the cull radius's 1e-5
+// relative margin. The profile's quotients are rounded once (quotient_by).
 __device__ __forceinline__ float lean_contribution(const CraterShapeKernel& k,
                                                    const LeanKernel& lk, const LeanCrater& l,
                                                    float dx, float dy, bool& reached) {
