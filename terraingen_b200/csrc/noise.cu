@@ -677,12 +677,12 @@ constexpr double kTurn3d[3][3] = {
     {0.7897926788435601, -0.24097777005594262, 0.5640542870894418},
     {0.011228581128535142, 0.9251190369776896, 0.37951111497202883}};
 
-constexpr int kBodyOctaves = kMaxFractals * (kMaxOctaves + 3 * kWarpOctaves);
 struct BodyOctave {
     double frequency;
     uint32_t seed, key;  // pcg(seed)
     float ox, oy, oz;
 };
+template <int kTurns, int kBodyOctaves>
 struct BodyLayout {
     uint32_t count;  // enabled fractals, in order
     struct {
@@ -691,9 +691,13 @@ struct BodyLayout {
         uint16_t first, warp;  // its octaves; its warp's 3 kWarpOctaves
         float amplitude, gain, offset, warpAmplitude;
     } fractals[kMaxFractals];
-    double turn[kMaxOctaves][9];  // an octave's turn, the same for every fractal
+    double turn[kTurns][9];  // an octave's turn, the same for every fractal
     BodyOctave octaves[kBodyOctaves];
 };
+// Any stack, and one of few octaves: a launch's arguments are copied with it, and 14 KB of them and
+// 32 turns made on the host took 1.5 us of a call of 17.5 (129^2 cells); with 3 KB and 16 turns they take 0.1.
+using FullBody = BodyLayout<kMaxOctaves, kMaxFractals * (kMaxOctaves + 3 * kWarpOctaves)>;
+using SmallBody = BodyLayout<16, 48>;
 
 // gradient3's sixteen directions as coefficients: two of x, y, z with signs, so their sum with
 // multiply-adds rounds once, as gradient3's u + v.
@@ -733,7 +737,8 @@ __device__ __forceinline__ float perlin3_table(const noise::Cell3& c, uint32_t k
 
 // Fractal3's octaves (fractal.h:284-316) at a point: world coordinates in double, each octave's
 // lattice point split in double before narrowing.
-__device__ __forceinline__ noise::Sums body_octaves(const BodyLayout& stack, uint32_t first,
+template <typename Layout>
+__device__ __forceinline__ noise::Sums body_octaves(const Layout& stack, uint32_t first,
                                                     int octaves, uint32_t basis, uint32_t type,
                                                     float gain, float offset, double x, double y,
                                                     double z, const float4* directions) {
@@ -764,8 +769,9 @@ __device__ __forceinline__ noise::Sums body_octaves(const BodyLayout& stack, uin
 // multiplied its own matrices, 120 with the host's, 82 with the corners' directions from a table
 // (calls of 81.3 us with room for seven blocks an SM, 82.5 without that bound, 83 to 85 with eight
 // to ten).
+template <typename Layout>
 __global__ void __launch_bounds__(128, 7)
-    noise_body_kernel(const __grid_constant__ BodyLayout stack, float elevation, uint32_t width,
+    noise_body_kernel(const __grid_constant__ Layout stack, float elevation, uint32_t width,
                       uint32_t height, const double* __restrict__ lons,
                       const double* __restrict__ lats, double radius,
                       float* __restrict__ heights) {
@@ -825,9 +831,10 @@ void host_body_octaves(BodyOctave* out, uint32_t seed, float wavelength, float l
     }
 }
 
-bool body_layout(const FractalStack& stack, BodyLayout& out) {
+template <int kTurns, int kBodyOctaves>
+bool body_layout(const FractalStack& stack, BodyLayout<kTurns, kBodyOctaves>& out) {
     double t[9] = {1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0};
-    for (int o = 0; o < kMaxOctaves; ++o) {
+    for (int o = 0; o < kTurns; ++o) {
         double next[9];
         for (int r = 0; r < 3; ++r) {
             for (int c = 0; c < 3; ++c) {
@@ -881,16 +888,26 @@ cudaError_t launch_noise_body(const FractalStack& stack, float elevation, uint32
     if (width == 0 || height == 0) {
         return cudaSuccess;
     }
-    static_assert(sizeof(BodyLayout) < 16384, "a kernel argument");
-    BodyLayout layout;
-    if (!body_layout(stack, layout)) {
-        return cudaErrorInvalidValue;
-    }
+    static_assert(sizeof(FullBody) < 16384, "a kernel argument");
     const dim3 block(32, 4);
     const dim3 grid((width + 31) / 32, (height + 3) / 4);
-    noise_body_kernel<<<grid, block, 0, stream>>>(layout, elevation, width, height, lons, lats,
-                                                  radius, heights);
-    return cudaGetLastError();
+    int deepest = kWarpOctaves, octaves = 0;
+    for (uint32_t i = 0; i < stack.count && i < kMaxFractals; ++i) {
+        const Fractal& f = stack.fractals[i];
+        if (f.enabled) {
+            deepest = std::max(deepest, int(f.octaves));
+            octaves += f.octaves + (f.warpAmplitude > 0.0f ? 3 * kWarpOctaves : 0);
+        }
+    }
+    auto launch = [&](auto layout) {
+        if (!body_layout(stack, layout)) {
+            return cudaErrorInvalidValue;
+        }
+        noise_body_kernel<<<grid, block, 0, stream>>>(layout, elevation, width, height, lons, lats,
+                                                      radius, heights);
+        return cudaGetLastError();
+    };
+    return deepest <= 16 && octaves <= 48 ? launch(SmallBody{}) : launch(FullBody{});
 }
 
 cudaError_t launch_noise(const FractalStack& stack, const Grid& grid, const Positions& at,
