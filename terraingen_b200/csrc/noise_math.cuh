@@ -234,7 +234,7 @@ __device__ __forceinline__ WorleyD worley2_within(const Cell2& c, uint32_t seed,
 // and is left out: 9 hashes for most points instead of 25. A second nearest at 1 or more is looked
 // for in the ring alone where the nearest is below 1 (no point of the ring can be nearest then), so
 // no point costs more than the 25 (F2 of 2 m cells on 1025^2 points of 0.5 m: 147 us with 25 for
-// every point, 153 when such points began again, 113 now).
+// every point, 153 when such points began again, 115 now).
 __device__ __forceinline__ WorleyD worley2(float x, float y, uint32_t seed, bool second) {
     const Cell2 c = split2(x, y);
     WorleyD w = worley2_within(c, seed, 1);

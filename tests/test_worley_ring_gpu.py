@@ -70,3 +70,21 @@ def test_matches_all_cells(device, basis):
              5: (f2 - f1) * F(0.447213595499957939)}[basis]
         want = F(2.0) * np.minimum(d, F(1.0)) - F(1.0)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("basis", [0, 1, 2, 3, 6])
+def test_a_stack_that_reads_second_nearest_points_changes_no_other_basis(device, basis):
+    """The kernel with that search and the one without."""
+    grid = N.Grid(97, 45, 10.0, 0.7, 0.0, 5.0, 0.0, -0.7)
+    one = fractal(seed=9, wavelength=20.0, amplitude=7.0, octaves=4, basis=basis, type=1)
+    outs = []
+    for other in (1, 4, 5):
+        f = np.array([one, fractal(seed=4, wavelength=50.0, amplitude=0.0, octaves=1,
+                                   basis=other)])
+        out = np.zeros((45, 97), np.float32)
+        N.check(device._lib.tg_noise_source(device._handle, f.ctypes.data, 2, 0.0, C.byref(grid),
+                                            out.ctypes.data, N.TG_MEMORY_HOST, None))
+        outs.append(out)
+    assert np.ptp(outs[0]) > 0.0
+    np.testing.assert_array_equal(outs[1], outs[0])
+    np.testing.assert_array_equal(outs[2], outs[0])
