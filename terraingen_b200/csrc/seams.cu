@@ -1382,6 +1382,7 @@ struct Solver {
     int order;
     cudaStream_t s;
     int sweeps, coarsest;
+    bool thin;             // the coarsest level has no post whose coarser one is whole
     const CgState* cg;     // the device state iterations stop on (null: always run)
     cudaStream_t capture;  // a stream of the library's own, the iterations are captured on
 };
@@ -1393,14 +1394,18 @@ struct Solver {
 // wide, with 2 sweeps, 12 iterations (14 with damped Jacobi sweeps) and 25 (46), within one of the
 // best fraction; here the three links of 2 x 2 patches with a 64-post overlap take 11 each on 5121^2
 // cells (Height) and 24, 22 and 41 on 2049^2 (Slope). The coarsest level takes all of them that n
-// sweeps can reduce, the largest over 3/4 n^2 and up.
-Chebyshev smoothing(const LevelView& L, int order, int sweeps, bool coarsest) {
+// sweeps can reduce, the largest over 3/4 n^2 and up; unless it is thin, without four unknowns whose
+// coarser post is whole: then none lies far below those of a gap two posts wide, the screening and
+// one neighbor's coupling, and n sweeps all but solve it (a gap of one column in nine: 2 iterations
+// for 10, 0.84 ms for 1.45 on 2000 x 1500 posts; 1.58 with damped Jacobi sweeps on four levels).
+Chebyshev smoothing(const LevelView& L, int order, int sweeps, bool coarsest, bool thin) {
     const double widest = L.center + 2.0 * L.cx + 2.0 * L.cy;
     const double least = L.center - 2.0 * L.cx - 2.0 * L.cy;
     const double high = order == 1 ? widest : widest * widest;
     double low;
     if (coarsest) {
-        low = std::max(order == 1 ? least : least * least,
+        const double floor = least + (thin ? std::min(L.cx, L.cy) : 0.0);
+        low = std::max(order == 1 ? floor : floor * floor,
                        high / std::max(0.75 * sweeps * sweeps, 3.0));
     } else {
         low = high / ((order == 1 ? 3.0 : 8.0) * sweeps);
@@ -1416,7 +1421,7 @@ double* cg_dots(CgState* cg) {
 // lands in x or, for sweeps from x with an odd count, in t.
 template <int kOrder, typename T>
 cudaError_t sweep(const Solver& sv, Level& L, int sweeps, bool fromZero, int done, bool coarsest) {
-    const Chebyshev c = smoothing(L.view, kOrder, sweeps, coarsest);
+    const Chebyshev c = smoothing(L.view, kOrder, sweeps, coarsest, sv.thin);
     T* const x = static_cast<T*>(L.x.ptr);
     T* const t = static_cast<T*>(L.t.ptr);
     T* cur = fromZero ? (sweeps % 2 == 0 ? x : t) : x;  // where the iterate before sweep 0 stands
@@ -1471,7 +1476,7 @@ int vcycle(Solver& sv, int d, int smoothed = 0) {
         const uint32_t threads = std::min<uint32_t>(1024, (L.view.n + 31) / 32 * 32);
         TG_PDL(coarsest_kernel<kOrder>, 1, threads, size_t(L.view.n) * 16, sv.s,
             L.view, static_cast<const double*>(L.b.ptr), static_cast<double*>(L.x.ptr),
-            smoothing(L.view, kOrder, sweeps, true), sweeps, sv.cg);
+            smoothing(L.view, kOrder, sweeps, true, sv.thin), sweeps, sv.cg);
         TG_CUDA(cudaGetLastError(), "coarsest launch");
         return TG_OK;
     }
@@ -1587,7 +1592,7 @@ int iteration(Solver& sv, CgState* cg) {
         TG_CUDA(cudaGetLastError(), "iteration launch");
         return TG_OK;
     }
-    const float scale = float(smoothing(L0.view, kOrder, sv.sweeps, false).first().beta);
+    const float scale = float(smoothing(L0.view, kOrder, sv.sweeps, false, false).first().beta);
     TG_PDL(cg_update_kernel, blocks_for(n), 256, 0, sv.s,
         x, r, p, ap, n, static_cast<float*>(L0.b.ptr),
         static_cast<float*>(first_sweep_target(L0, sv.sweeps)), scale, cg);
@@ -1884,6 +1889,7 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
     const int order = o.mode == 3u ? 2 : 1;
     const double screening = 1.0 / (o.decay_length * o.decay_length);
     int levels = 0;
+    bool thin = false;
     uint32_t lw = width, lh = height, lp = pitch;
     double ldx = dx, ldy = dy;
     for (; levels < int(o.levels); ++levels) {
@@ -1914,6 +1920,7 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
             return finish(TG_OK);
         }
         if (L.view.n == 0) {
+            thin = true;
             break;  // no whole coarse post: the level before is the coarsest
         }
         if (L.view.n <= 32u || lw < 4 || lh < 4) {  // the coarsest, as kCoarsestPosts
@@ -1985,7 +1992,8 @@ int tg_seam_solve(tg_device* d, const uint8_t* data, const float* difference, ui
                                      int(kCoarsestBlockPosts * 16)),
                 "shared memory attribute");
     }
-    Solver sv{&wk, levels, order, s, int(o.sweeps), int(o.coarsest_sweeps), nullptr, d->stream};
+    Solver sv{&wk,  levels,  order,    s, int(o.sweeps), int(o.coarsest_sweeps),
+              thin, nullptr, d->stream};
     int iterations = 0;
     const double tolerance = o.tolerance > 0.0 ? o.tolerance : 1e-10;
     const int st = order == 1 ? solve<1>(sv, tolerance, 200, &iterations)
